@@ -476,6 +476,351 @@ __global__ void __launch_bounds__(kChiBlock, 3) chi_terms_hoisted_kernel(const C
     }
 }
 
+// ---------------------------------------------------------------------------
+// the factored kernel
+// ---------------------------------------------------------------------------
+// The four c+ elements of a term form a cycle i - x - m - y - i, and every Phi
+// splits into factors of at most two energies, so the sum over (j, k, l) is a
+// chain of small matrix products instead of a loop over all triples:
+//   phi_ki, phi_li  (m = k, m = j):  sum_m M_m (sum_x A_ix X_x B_xm) (sum_y C_my Y_y D_yi)
+//   phi_ji  (x = k, m = l, y = j):   sum_m [T_m sum_x A_ix (B a)_xm - p_m sum_x A_ix K_x (B a)_xm],
+//                                    p_m = sum_y C_my b_y D_yi  (T_m = L_m p_m, or the same with
+//                                    b^2 - beta b where the denominator vanishes)
+//   phi_ii  (x = j, m = k, y = l):   sum_xy A_ix t_xy G_xy D_yi - sum_m [sum_x A_ix (B c)_xm (b_x + K_m)] (C a D)_mi,
+//                                    G = B (C a) once for all i
+// with the same one- and two-index inverses and the same branches as phi_*.
+// O(n^3) operations per (term, triple) against O(n^4) one by one: 512 triples
+// of the ns = 4 (2,2) sector (36 states) take 2.1 ms a call, 130.6 ms with the
+// split kernel above.
+// One block per (term, triple), its tables in shared memory (five of n (n | 1)
+// complex numbers, 107 KB at n = 36: two blocks per SM) or, for larger
+// sectors, in a slice of global memory; a thread owns two states i and one of
+// the cycle's other indices, so one table element serves both states.  FP64
+// arithmetic and shared-memory loads bound it about equally.
+struct FacTerm {
+    int op, nphi, kind[2], perm[2][3], sgn[2], total;
+    int sx, sm, sy;           // sectors of x, m, y
+    int64_t off[4];           // factors (i,x), (x,m), (m,y), (y,i)
+    int s0[4], s1[4];         // strides of the pair's first and second index
+};
+
+// |z| > eps, rounded the same wherever it is evaluated
+__device__ __forceinline__ bool above_rn(Cx z, double eps2)
+{
+    return __dadd_rn(__dmul_rn(z.re, z.re), __dmul_rn(z.im, z.im)) > eps2;
+}
+
+// the roles (x, m, y) of (j, k, l) for a Phi kernel, as variables
+__host__ __device__ inline void fac_roles(int kind, int (&v)[3])
+{
+    if (kind == P_JI) { v[0] = VK; v[1] = VL; v[2] = VJ; }
+    else if (kind == P_LI) { v[0] = VK; v[1] = VJ; v[2] = VL; }
+    else { v[0] = VJ; v[1] = VK; v[2] = VL; }
+}
+
+// acc[i] += sgn * sum over e < n of R[i * ld + e], one warp per state, in a fixed order
+__device__ __forceinline__ void fac_reduce(const Cx *R, int ld, int n, int ni, double sgn, Cx *acc)
+{
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int i = threadIdx.x >> 5; i < ni; i += blockDim.x >> 5) {
+        Cx t = cx(0.0);
+        for (int e = lane; e < n; e += 32) t = t + R[i * ld + e];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            t.re += __shfl_down_sync(0xffffffffu, t.re, o);
+            t.im += __shfl_down_sync(0xffffffffu, t.im, o);
+        }
+        if (lane == 0) acc[i] = acc[i] + t * sgn;
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(kChiBlock, 2) chi_factored_kernel(const ChiArgs A, const FacTerm *terms, const double *boltz,
+                                                                    int nmax, Cx *ws, int64_t nitem)
+{
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    __shared__ int s_any;
+    Cx *base = ws ? ws + (int64_t)blockIdx.x * 5 * nmax * (nmax | 1) : reinterpret_cast<Cx *>(sm_raw);
+    Cx *acc = reinterpret_cast<Cx *>(sm_raw) + (ws ? 0 : 5 * nmax * (nmax | 1));
+    Cx *tab[5];
+#pragma unroll
+    for (int q = 0; q < 5; ++q) tab[q] = base + (int64_t)q * nmax * (nmax | 1);
+    const int tid = threadIdx.x, nt = blockDim.x, ni = A.ni, np = (ni + 1) / 2;
+    const double eps2 = A.eps * A.eps, beta = A.beta;
+    const double *Ei = A.E + A.eoff[S_I];
+    for (int64_t item = blockIdx.x; item < nitem; item += gridDim.x) {
+        const int f = (int)(item / A.nterm), t = (int)(item % A.nterm);
+        const FacTerm &T = terms[t];
+        const int dx = A.dim[T.sx], dm = A.dim[T.sm], dy = A.dim[T.sy];
+        const int lx = dx | 1, lm = dm | 1, ly = dy | 1;
+        const double *Ex = A.E + A.eoff[T.sx], *Em = A.E + A.eoff[T.sm], *Ey = A.E + A.eoff[T.sy];
+        const double *Aix = A.C + T.off[0], *Bxm = A.C + T.off[1], *Cmy = A.C + T.off[2], *Dyi = A.C + T.off[3];
+        const int a0 = T.s0[0], a1 = T.s1[0], b0 = T.s0[1], b1 = T.s1[1], c0 = T.s0[2], c1 = T.s1[2], d0 = T.s0[3],
+                  d1 = T.s1[3];
+        const Cx w[3] = {Cx{A.w[6 * f], A.w[6 * f + 1]}, Cx{A.w[6 * f + 2], A.w[6 * f + 3]},
+                         Cx{A.w[6 * f + 4], A.w[6 * f + 5]}};
+        __syncthreads();
+        for (int i = tid; i < ni; i += nt) acc[i] = cx(0.0);
+        for (int ev = 0; ev < T.nphi; ++ev) {
+            const Cx W1 = w[T.perm[ev][0]], W2 = w[T.perm[ev][1]], W3 = w[T.perm[ev][2]];
+            const Cx Ws12 = W1 + W2, Ws23 = W2 + W3, Ws123 = W1 + W2 + W3;
+            const double sgn = (double)(T.sgn[ev] * T.total);
+            const int kind = T.kind[ev];
+            Cx *R = tab[4];
+            __syncthreads();
+            if (kind == P_II) {
+                // x = j, m = k, y = l
+                Cx *Ca = tab[0], *G = tab[1], *Bc = tab[2], *bx = tab[3];
+                for (int e = tid; e < dm * dy; e += nt) {
+                    const int m = e / dy, y = e - m * dy;
+                    Ca[m * ly + y] = inv_fast(W3 + (Em[m] - Ey[y])) * __ldg(Cmy + (int64_t)c0 * m + (int64_t)c1 * y);
+                }
+                for (int e = tid; e < dx * dm; e += nt) {
+                    const int x = e / dm, m = e - x * dm;
+                    Bc[x * lm + m] = inv_fast(W2 + (Ex[x] - Em[m])) * __ldg(Bxm + (int64_t)b0 * x + (int64_t)b1 * m);
+                }
+                for (int e = tid; e < ni * dx; e += nt) {
+                    const int i = e / dx, x = e - i * dx;
+                    bx[i * lx + x] = inv_fast(W1 + (Ei[i] - Ex[x]));
+                }
+                if (tid == 0) s_any = 0;
+                __syncthreads();
+                // G = B (C a), times 1/z; where z vanishes G alone, marked by a table entry of its own
+                for (int e = tid; e < dx * dy; e += nt) {
+                    const int x = e / dy, y = e - x * dy;
+                    const double *bp = Bxm + (int64_t)b0 * x;
+                    Cx g = cx(0.0);
+                    for (int m = 0; m < dm; ++m) {
+                        const double b = __ldg(bp + (int64_t)b1 * m);
+                        const Cx c = Ca[m * ly + y];
+                        g.re = fma(b, c.re, g.re);
+                        g.im = fma(b, c.im, g.im);
+                    }
+                    const Cx z = Ws23 + (Ex[x] - Ey[y]);
+                    if (above_rn(z, eps2)) g = g * inv_fast(z);
+                    else s_any = 1;
+                    G[x * ly + y] = g;
+                }
+                __syncthreads();
+                const bool any = s_any != 0;
+                for (int e = tid; e < np * dy; e += nt) {
+                    const int ip = e / dy, y = e - ip * dy, i0 = 2 * ip, i1 = i0 + 1 < ni ? i0 + 1 : i0;
+                    const Cx L0 = inv_fast(Ws123 + (Ei[i0] - Ey[y])), L1 = inv_fast(Ws123 + (Ei[i1] - Ey[y]));
+                    Cx p0 = cx(0.0), p1 = cx(0.0);
+                    for (int x = 0; x < dx; ++x) {
+                        const Cx g = G[x * ly + y], u0 = bx[i0 * lx + x], u1 = bx[i1 * lx + x];
+                        Cx t0 = u0 - L0, t1 = u1 - L1;
+                        if (any && !above_rn(Ws23 + (Ex[x] - Ey[y]), eps2)) { t0 = u0 * u0; t1 = u1 * u1; }
+                        const double f0 = __ldg(Aix + (int64_t)a0 * i0 + (int64_t)a1 * x);
+                        const double f1 = __ldg(Aix + (int64_t)a0 * i1 + (int64_t)a1 * x);
+                        p0 = p0 + (g * t0) * f0;
+                        p1 = p1 + (g * t1) * f1;
+                    }
+                    R[i0 * ly + y] = p0 * __ldg(Dyi + (int64_t)d0 * y + (int64_t)d1 * i0);
+                    if (i1 > i0) R[i1 * ly + y] = p1 * __ldg(Dyi + (int64_t)d0 * y + (int64_t)d1 * i1);
+                }
+                fac_reduce(R, ly, dy, ni, sgn, acc);
+                for (int e = tid; e < np * dm; e += nt) {
+                    const int ip = e / dm, m = e - ip * dm, i0 = 2 * ip, i1 = i0 + 1 < ni ? i0 + 1 : i0;
+                    Cx p0 = cx(0.0), p1 = cx(0.0), q0 = cx(0.0), q1 = cx(0.0), r0 = cx(0.0), r1 = cx(0.0);
+                    for (int x = 0; x < dx; ++x) {
+                        const Cx b = Bc[x * lm + m];
+                        const Cx h0 = b * __ldg(Aix + (int64_t)a0 * i0 + (int64_t)a1 * x);
+                        const Cx h1 = b * __ldg(Aix + (int64_t)a0 * i1 + (int64_t)a1 * x);
+                        p0 = p0 + h0 * bx[i0 * lx + x];
+                        p1 = p1 + h1 * bx[i1 * lx + x];
+                        q0 = q0 + h0;
+                        q1 = q1 + h1;
+                    }
+                    for (int y = 0; y < dy; ++y) {
+                        const Cx c = Ca[m * ly + y];
+                        r0 = r0 + c * __ldg(Dyi + (int64_t)d0 * y + (int64_t)d1 * i0);
+                        r1 = r1 + c * __ldg(Dyi + (int64_t)d0 * y + (int64_t)d1 * i1);
+                    }
+                    const Cx y0 = Ws12 + (Ei[i0] - Em[m]), y1 = Ws12 + (Ei[i1] - Em[m]);
+                    const Cx K0 = above_rn(y0, eps2) ? -inv_fast(y0) : cx(beta);
+                    const Cx K1 = above_rn(y1, eps2) ? -inv_fast(y1) : cx(beta);
+                    R[i0 * lm + m] = (p0 + q0 * K0) * r0;
+                    if (i1 > i0) R[i1 * lm + m] = (p1 + q1 * K1) * r1;
+                }
+                fac_reduce(R, lm, dm, ni, -sgn, acc);
+            } else if (kind == P_JI) {
+                // x = k, m = l, y = j
+                Cx *Ba = tab[0], *by = tab[1], *Kx = tab[2];
+                double *Cm = reinterpret_cast<double *>(tab[3]);        // [y][m]
+                for (int e = tid; e < dx * dm; e += nt) {
+                    const int x = e / dm, m = e - x * dm;
+                    Ba[x * lm + m] = inv_fast(W3 + (Ex[x] - Em[m])) * __ldg(Bxm + (int64_t)b0 * x + (int64_t)b1 * m);
+                }
+                for (int e = tid; e < dy * dm; e += nt) {
+                    const int y = e / dm, m = e - y * dm;
+                    Cm[y * lm + m] = __ldg(Cmy + (int64_t)c0 * m + (int64_t)c1 * y);
+                }
+                for (int e = tid; e < ni * dy; e += nt) {
+                    const int i = e / dy, y = e - i * dy;
+                    by[i * ly + y] = inv_fast(W1 + (Ey[y] - Ei[i]));
+                }
+                for (int e = tid; e < ni * dx; e += nt) {
+                    const int i = e / dx, x = e - i * dx;
+                    Kx[i * lx + x] = inv_fast(W2 + (Ei[i] - Ex[x]));
+                }
+                __syncthreads();
+                for (int e = tid; e < np * dm; e += nt) {
+                    const int ip = e / dm, m = e - ip * dm, i0 = 2 * ip, i1 = i0 + 1 < ni ? i0 + 1 : i0;
+                    Cx X0 = cx(0.0), X1 = cx(0.0), Y0 = cx(0.0), Y1 = cx(0.0), p0 = cx(0.0), p1 = cx(0.0);
+                    for (int x = 0; x < dx; ++x) {
+                        const Cx b = Ba[x * lm + m];
+                        const Cx h0 = b * __ldg(Aix + (int64_t)a0 * i0 + (int64_t)a1 * x);
+                        const Cx h1 = b * __ldg(Aix + (int64_t)a0 * i1 + (int64_t)a1 * x);
+                        X0 = X0 + h0;
+                        X1 = X1 + h1;
+                        Y0 = Y0 + h0 * Kx[i0 * lx + x];
+                        Y1 = Y1 + h1 * Kx[i1 * lx + x];
+                    }
+                    for (int y = 0; y < dy; ++y) {
+                        const double c = Cm[y * lm + m];
+                        const double f0 = c * __ldg(Dyi + (int64_t)d0 * y + (int64_t)d1 * i0);
+                        const double f1 = c * __ldg(Dyi + (int64_t)d0 * y + (int64_t)d1 * i1);
+                        p0 = p0 + by[i0 * ly + y] * f0;
+                        p1 = p1 + by[i1 * ly + y] * f1;
+                    }
+                    const Cx z0 = Ws23 + (Ei[i0] - Em[m]), z1 = Ws23 + (Ei[i1] - Em[m]);
+                    const bool v0 = above_rn(z0, eps2), v1 = above_rn(z1, eps2);
+                    Cx T0 = p0 * inv_fast(v0 ? z0 : cx(1.0)), T1 = p1 * inv_fast(v1 ? z1 : cx(1.0));
+                    if (!v0 || !v1) {
+                        Cx g0 = cx(0.0), g1 = cx(0.0);
+                        for (int y = 0; y < dy; ++y) {
+                            const double c = Cm[y * lm + m];
+                            const Cx u0 = by[i0 * ly + y], u1 = by[i1 * ly + y];
+                            g0 = g0 + (u0 * u0 - u0 * beta) * (c * __ldg(Dyi + (int64_t)d0 * y + (int64_t)d1 * i0));
+                            g1 = g1 + (u1 * u1 - u1 * beta) * (c * __ldg(Dyi + (int64_t)d0 * y + (int64_t)d1 * i1));
+                        }
+                        if (!v0) T0 = g0;
+                        if (!v1) T1 = g1;
+                    }
+                    R[i0 * lm + m] = T0 * X0 - p0 * Y0;
+                    if (i1 > i0) R[i1 * lm + m] = T1 * X1 - p1 * Y1;
+                }
+                fac_reduce(R, lm, dm, ni, sgn, acc);
+            } else {
+                // phi_ki: x = j, m = k, y = l;  phi_li: x = k, m = j, y = l
+                const bool ki = kind == P_KI;
+                double *Bm = reinterpret_cast<double *>(tab[0]);        // [x][m]
+                double *Cm = reinterpret_cast<double *>(tab[1]);        // [y][m]
+                Cx *Px = tab[2], *Qy = tab[3];
+                for (int e = tid; e < dx * dm; e += nt) {
+                    const int x = e / dm, m = e - x * dm;
+                    Bm[x * lm + m] = __ldg(Bxm + (int64_t)b0 * x + (int64_t)b1 * m);
+                }
+                for (int e = tid; e < dy * dm; e += nt) {
+                    const int y = e / dm, m = e - y * dm;
+                    Cm[y * lm + m] = __ldg(Cmy + (int64_t)c0 * m + (int64_t)c1 * y);
+                }
+                const Cx Wx = ki ? W2 : W3;
+                for (int e = tid; e < ni * dx; e += nt) {
+                    const int i = e / dx, x = e - i * dx;
+                    Px[i * lx + x] = inv_fast(Wx + (Ex[x] - Ei[i])) * __ldg(Aix + (int64_t)a0 * i + (int64_t)a1 * x);
+                }
+                for (int e = tid; e < ni * dy; e += nt) {
+                    const int i = e / dy, y = e - i * dy;
+                    Qy[i * ly + y] = inv_fast(ki ? W3 + (Ei[i] - Ey[y]) : Ws123 + (Ey[y] - Ei[i])) *
+                                     __ldg(Dyi + (int64_t)d0 * y + (int64_t)d1 * i);
+                }
+                __syncthreads();
+                const Cx Wm = ki ? Ws12 : Ws23;
+                for (int e = tid; e < np * dm; e += nt) {
+                    const int ip = e / dm, m = e - ip * dm, i0 = 2 * ip, i1 = i0 + 1 < ni ? i0 + 1 : i0;
+                    Cx u0 = cx(0.0), u1 = cx(0.0), v0 = cx(0.0), v1 = cx(0.0);
+                    for (int x = 0; x < dx; ++x) {
+                        const double b = Bm[x * lm + m];
+                        u0 = u0 + Px[i0 * lx + x] * b;
+                        u1 = u1 + Px[i1 * lx + x] * b;
+                    }
+                    for (int y = 0; y < dy; ++y) {
+                        const double c = Cm[y * lm + m];
+                        v0 = v0 + Qy[i0 * ly + y] * c;
+                        v1 = v1 + Qy[i1 * ly + y] * c;
+                    }
+                    const Cx z0 = Wm + (Em[m] - Ei[i0]), z1 = Wm + (Em[m] - Ei[i1]);
+                    R[i0 * lm + m] = above_rn(z0, eps2) ? -(u0 * v0 * inv_fast(z0)) : cx(0.0);
+                    if (i1 > i0) R[i1 * lm + m] = above_rn(z1, eps2) ? -(u1 * v1 * inv_fast(z1)) : cx(0.0);
+                }
+                fac_reduce(R, lm, dm, ni, sgn, acc);
+            }
+        }
+        // the Boltzmann-weighted sum over the states, in a fixed order
+        __syncthreads();
+        if (tid < 32) {
+            Cx s = cx(0.0);
+            for (int i = tid; i < ni; i += 32) s = s + acc[i] * __ldg(boltz + i);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                s.re += __shfl_down_sync(0xffffffffu, s.re, o);
+                s.im += __shfl_down_sync(0xffffffffu, s.im, o);
+            }
+            if (tid == 0) {
+                A.part[item * 2] = s.re;
+                A.part[item * 2 + 1] = s.im;
+            }
+        }
+    }
+}
+
+// out[op - 1][f] = the sum of the triple's terms of that operator pair, in table order.
+__global__ void chi_factored_sum_kernel(const ChiArgs A, const FacTerm *terms, double *out)
+{
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= A.nf) return;
+    Cx s[2] = {cx(0.0), cx(0.0)};
+    const double2 *p = reinterpret_cast<const double2 *>(A.part) + (int64_t)f * A.nterm;
+    for (int t = 0; t < A.nterm; ++t) {
+        const double2 v = p[t];
+        Cx &o = s[terms[t].op - 1];
+        o.re += v.x;
+        o.im += v.y;
+    }
+    for (int q = 0; q < 2; ++q) {
+        out[2 * ((int64_t)q * A.nf + f)] = s[q].re;
+        out[2 * ((int64_t)q * A.nf + f) + 1] = s[q].im;
+    }
+}
+
+// The factored form of a term; false when its factors are no such cycle.
+bool factor_term(const DevTerm &d, const ChiArgs &A, FacTerm &o)
+{
+    int v[3];
+    fac_roles(d.kind[0], v);
+    if (d.nphi == 2) {
+        int v2[3];
+        fac_roles(d.kind[1], v2);
+        if (v2[0] != v[0] || v2[1] != v[1] || v2[2] != v[2]) return false;
+    }
+    const int sec[4] = {S_I, d.sj, d.sk, d.sl};
+    o.op = d.op; o.nphi = d.nphi; o.total = d.total;
+    for (int q = 0; q < 2; ++q) {
+        o.kind[q] = d.kind[q];
+        o.sgn[q] = d.sgn[q];
+        for (int r = 0; r < 3; ++r) o.perm[q][r] = d.perm[q][r];
+    }
+    o.sx = sec[v[0]]; o.sm = sec[v[1]]; o.sy = sec[v[2]];
+    const int pair[4][2] = {{VI, v[0]}, {v[0], v[1]}, {v[1], v[2]}, {v[2], VI}};
+    for (int p = 0; p < 4; ++p) {
+        int found = -1;
+        for (int q = 0; q < 4; ++q)
+            if ((d.row[q] == pair[p][0] && d.col[q] == pair[p][1]) || (d.row[q] == pair[p][1] && d.col[q] == pair[p][0])) {
+                if (found >= 0) return false;
+                found = q;
+            }
+        if (found < 0) return false;
+        o.off[p] = A.moff[d.mat[found]];
+        const bool straight = d.row[found] == pair[p][0];
+        o.s0[p] = straight ? d.ld[found] : 1;
+        o.s1[p] = straight ? 1 : d.ld[found];
+    }
+    return true;
+}
+
 // out[f] = sum_i boltz_i sum_t part[f][t][i] for the terms of one op, in order.
 __global__ void chi_reduce_kernel(const ChiArgs A, const double *boltz, int op, double *out)
 {
@@ -526,8 +871,89 @@ int edk_chiloc_set_kernel(int plain)
 }
 
 int edk_internal_fail(edk_ctx *ctx, int code, const char *msg);
+void *edk_internal_scratch(edk_ctx *ctx, int slot, size_t bytes);
+void edk_internal_scratch_done(edk_ctx *ctx);
+int edk_internal_num_sms(const edk_ctx *ctx);
 void edk_internal_add_launches(edk_ctx *ctx, int64_t n);
 void edk_internal_count(edk_ctx *ctx, int64_t h2d, int64_t d2h);
+
+static constexpr int kNotFactored = -1;
+
+// The factored kernel for all terms and triples; kNotFactored where it does
+// not apply: a frequency (or the sum of the three) within 1e-8 of the real
+// axis, whose inverses may overflow and which the element-by-element kernels
+// only evaluate where the matrix elements are non-zero, or no memory.
+static int chiloc_factored(edk_ctx *ctx, const ChiArgs &A_in, const std::vector<DevTerm> &terms,
+                           const std::vector<double> &E, const std::vector<double> &C,
+                           const std::vector<double> &boltz, const double *w, double *out1, double *out2)
+{
+    ChiArgs A = A_in;
+    for (int f = 0; f < A.nf; ++f) {
+        const double *q = w + (size_t)f * 6;
+        const double im[4] = {q[1], q[3], q[5], q[1] + q[3] + q[5]};
+        for (double v : im)
+            if (!(std::fabs(v) >= 1e-8)) return kNotFactored;
+    }
+    std::vector<FacTerm> ft(terms.size());
+    int nmax = A.ni;
+    for (size_t t = 0; t < terms.size(); ++t) {
+        if (!factor_term(terms[t], A, ft[t])) return kNotFactored;
+        nmax = std::max({nmax, A.dim[ft[t].sx], A.dim[ft[t].sm], A.dim[ft[t].sy]});
+    }
+    cudaStream_t st = edk_internal_stream(ctx);
+    // one upload: energies, matrices, weights, frequencies, terms
+    const size_t nE = E.size(), nC = C.size(), nB = boltz.size(), nW = (size_t)A.nf * 6;
+    const size_t nT = (ft.size() * sizeof(FacTerm) + 7) / 8, nIn = nE + nC + nB + nW + nT;
+    const size_t nOut = (size_t)A.nf * 4;
+    std::vector<double> in(nIn);
+    double *h = in.data();
+    std::copy(E.begin(), E.end(), h);
+    std::copy(C.begin(), C.end(), h + nE);
+    std::copy(boltz.begin(), boltz.end(), h + nE + nC);
+    std::copy(w, w + nW, h + nE + nC + nB);
+    std::memcpy(h + nE + nC + nB + nW, ft.data(), ft.size() * sizeof(FacTerm));
+    const int64_t nitem = (int64_t)A.nf * A.nterm;
+    double *d = static_cast<double *>(edk_internal_scratch(ctx, 0, (nIn + nOut) * 8));
+    double *part = static_cast<double *>(edk_internal_scratch(ctx, 1, (size_t)nitem * 16));
+    if (!d || !part) return kNotFactored;
+    // the tables: in shared memory up to two blocks per SM, else in slices of
+    // at most 2 GB of global memory
+    const size_t tab = (size_t)5 * nmax * (nmax | 1) * sizeof(Cx);
+    const bool in_smem = tab + sizeof(Cx) * A.ni <= 110 * 1024;
+    const size_t smem = (in_smem ? tab : 0) + sizeof(Cx) * A.ni;
+    if (smem > 200 * 1024) return kNotFactored;
+    int64_t grid = (int64_t)edk_internal_num_sms(ctx) * 2;
+    Cx *ws = nullptr;
+    if (!in_smem) {
+        grid = std::min<int64_t>(grid, std::max<int64_t>(1, (int64_t)(((size_t)2 << 30) / tab)));
+        ws = static_cast<Cx *>(edk_internal_scratch(ctx, 2, tab * (size_t)grid));
+        if (!ws) return kNotFactored;
+    }
+    grid = std::min(grid, nitem);
+    cudaError_t e = cudaMemcpyAsync(d, h, nIn * 8, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(chi_factored_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) {
+        A.E = d;
+        A.C = d + nE;
+        A.w = d + nE + nC + nB;
+        A.part = part;
+        const FacTerm *dt = reinterpret_cast<const FacTerm *>(d + nE + nC + nB + nW);
+        chi_factored_kernel<<<(int)grid, kChiBlock, smem, st>>>(A, dt, d + nE + nC, nmax, ws, nitem);
+        chi_factored_sum_kernel<<<(A.nf + 63) / 64, 64, 0, st>>>(A, dt, d + nIn);
+        e = cudaGetLastError();
+        edk_internal_add_launches(ctx, 2);
+    }
+    for (int op = 0; op < 2 && e == cudaSuccess; ++op)
+        if (double *o = op == 0 ? out1 : out2)
+            e = cudaMemcpyAsync(o, d + nIn + (size_t)op * 2 * A.nf, sizeof(double) * 2 * A.nf, cudaMemcpyDeviceToHost,
+                                st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return edk_internal_fail(ctx, EDK_ERR_CUDA, cudaGetErrorString(e));
+    edk_internal_scratch_done(ctx);
+    edk_internal_count(ctx, (int64_t)(nIn - nT) * 8, (int64_t)A.nf * 16 * ((out1 ? 1 : 0) + (out2 ? 1 : 0)));
+    return EDK_OK;
+}
 
 int edk_chiloc(edk_ctx *ctx, int32_t op_mask, double beta, double Z, double gs_e, double phi_eps, int32_t sites,
                int32_t nup, int32_t ndn, const edk_chiloc_sectors *s, int32_t nf, const double *w_host,
@@ -587,6 +1013,16 @@ int edk_chiloc(edk_ctx *ctx, int32_t op_mask, double beta, double Z, double gs_e
     for (int i = 0; i < ni; ++i) boltz[i] = std::exp(-(s->E[S_I][i] - gs_e) * beta) / Z;
     cudaStream_t st = edk_internal_stream(ctx);
     const int nterm = (int)terms.size();
+    A.nterm = nterm;
+    A.ni = ni;
+    A.nf = nf;
+    A.beta = beta;
+    A.eps = phi_eps;
+    if (!chiloc_plain_kernel && nterm > 0) {
+        const int rc = chiloc_factored(ctx, A, terms, E, C, boltz, w_host, (op_mask & 1) ? pdndn_host : nullptr,
+                                       (op_mask & 2) ? pupdn_host : nullptr);
+        if (rc != kNotFactored) return rc;
+    }
     DevMem dE, dC, dT, dW, dP, dB, dO;
     cudaError_t e;
     if ((e = put(dE, E.data(), E.size(), st)) != cudaSuccess || (e = put(dC, C.data(), C.size(), st)) != cudaSuccess ||
@@ -598,11 +1034,6 @@ int edk_chiloc(edk_ctx *ctx, int32_t op_mask, double beta, double Z, double gs_e
         return edk_internal_fail(ctx, e == cudaErrorMemoryAllocation ? EDK_ERR_NOMEM : EDK_ERR_CUDA,
                                  cudaGetErrorString(e));
     edk_internal_count(ctx, (int64_t)(E.size() + C.size() + (size_t)nf * 6 + boltz.size()) * 8, 0);
-    A.nterm = nterm;
-    A.ni = ni;
-    A.nf = nf;
-    A.beta = beta;
-    A.eps = phi_eps;
     A.E = static_cast<const double *>(dE.p);
     A.C = static_cast<const double *>(dC.p);
     A.terms = static_cast<const DevTerm *>(dT.p);

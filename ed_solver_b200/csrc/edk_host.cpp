@@ -120,6 +120,9 @@ struct edk_ctx {
     // per-block workspace, and the autotuned launch shape per problem class
     DevBuf b_hams, b_items, b_queue, b_alpha, b_beta, b_done, b_work;
     DevBuf tile_scratch;      // partial sums of the two-pass row step (kind 5)
+    // buffers of the other drivers (edk_internal_scratch), at most 256 MB each
+    // between calls; edk_ctx_trim gives them back
+    DevBuf scratch[3];
     struct BatchShape { int block, R, per_sm; };
     std::vector<std::pair<std::string, BatchShape>> batch_tuned;
     // fast-kernel launch shape timed per sector shape (element type, dim_up,
@@ -1033,6 +1036,28 @@ void edk_internal_fp32_sums(edk_ctx *ctx, int *enable, int64_t *min_dim)
     *min_dim = ctx->fp32_sums_min_dim;
 }
 
+int edk_internal_num_sms(const edk_ctx *ctx) { return ctx->num_sms; }
+
+// A buffer of at least `bytes` for work on the context's stream, null when
+// there is no memory for it.  It holds until the next request for the slot.
+void *edk_internal_scratch(edk_ctx *ctx, int slot, size_t bytes)
+{
+    DevBuf &b = ctx->scratch[slot];
+    if (b.ensure(bytes) == cudaSuccess) return b.p;
+    (void)cudaGetLastError();
+    b.p = nullptr;
+    b.bytes = 0;
+    return nullptr;
+}
+
+// After a call has synchronised: buffers above 256 MB are given back, the
+// others stay for the next call.
+void edk_internal_scratch_done(edk_ctx *ctx)
+{
+    for (DevBuf &b : ctx->scratch)
+        if (b.bytes > (size_t)256 << 20) b.release();
+}
+
 int edk_internal_fail(edk_ctx *ctx, int code, const char *msg) { return ctx->fail(code, "%s", msg); }
 
 edk_ctx *edk_internal_h_ctx(edk_h *h) { return h->ctx; }
@@ -1129,9 +1154,10 @@ int edk_ctx_set_fp32_sums(edk_ctx *ctx, int enable, int64_t min_dim)
 int edk_ctx_trim(edk_ctx *ctx)
 {
     if (!ctx) return EDK_ERR_INVALID;
-    if (!ctx->basis_pool) return EDK_OK;
     int rc = ctx->cuda(cudaStreamSynchronize(ctx->stream), "sync");
     if (rc) return rc;
+    for (DevBuf &b : ctx->scratch) b.release();
+    if (!ctx->basis_pool) return EDK_OK;
     return ctx->cuda(cudaMemPoolTrimTo(ctx->basis_pool, 0), "cudaMemPoolTrimTo");
 }
 
