@@ -208,8 +208,9 @@ struct SzTerm {
 // low half (up-up), 1 = both in the high half (hole-hole), 2 = one in each
 // (pairing).  Up-up runs carry a table over the low halves: for low-half
 // position p (low_states order) entry k at ell[ell_off + k*2^ns + p] is the
-// k-th active term's target rank_low (16 bits) | sign (bit 16) | index in the
-// run (bits 17..31), or 0xFFFFFFFF after the last.
+// k-th active term's target rank_low (16 bits) | byte offset of its signed
+// value, (2 * term + sign) * 8, in bits 16..31; after the last the state's own
+// rank_low | (2 * terms) * 8 << 16.  Popcount class k has at most kell[k*nrun + run].
 struct SzRun {
     int32_t kind, first, count, kell;
     int64_t ell_off;
@@ -217,8 +218,9 @@ struct SzRun {
 
 struct SzSectorDev {
     int npart = 0, nrows = 0, maxlen = 0;
+    int pitch = 0;                     // longest class of a row or one particle away from it, rounded up to 4
     int64_t dim = 0;
-    const uint32_t *row_h = nullptr;   // nrows high halves present in the sector, ascending
+    const uint32_t *row_h = nullptr;   // nrows high halves present in the sector, in processing order
     const uint32_t *off_h = nullptr;   // 2^ns: rank of the first state of high half h
 };
 
@@ -240,7 +242,20 @@ struct SzDev {
     const SzRun *runs = nullptr;
     const int32_t *term_run = nullptr;      // nterm: run of each term
     const uint32_t *ell = nullptr;          // the up-up runs' tables
+    // Diagonal sum through the up baths (up impurity, hole impurity, up baths:
+    // the order of the tabulated form), per hole-impurity configuration and
+    // low-half position: pdiag[cfg * 2^ns + p].  Tabulated order only.
+    const double *pdiag = nullptr;
+    // Per low orbital o of a pairing term, table pair_row[o]: for low-half
+    // position p, rank_low of the state with o flipped | parity of the occupied
+    // orbitals above o << 16 | occupation of o << 17.
+    const uint32_t *pair = nullptr;
+    const uint32_t *kell = nullptr;         // longest entry list per popcount class and run
+    uint8_t pair_row[16] = {0}, pair_orb[16] = {0};   // table of an orbital, orbital of a table
+    uint32_t smem_lists = 0;                // bytes of a row's lists in shared memory
 };
+
+cudaError_t launch_sz_pair(const SzDev &S, int nrow, uint32_t *pair, cudaStream_t st);
 
 struct SzHost;   // host tables and device copies of one Nambu sector (edk_sz.cpp)
 int sz_create(const edk_model_sz *m, int npart, cudaStream_t st, SzHost **out, std::string *err);
