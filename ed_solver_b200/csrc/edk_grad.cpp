@@ -9,7 +9,7 @@
 //       w_k = H v_k - b_k v_{k-1},  a_k = <w_k, v_k>,  r_k = w_k - a_k v_k,
 //       b_{k+1} = |r_k|,  v_{k+1} = r_k / b_{k+1}.
 //     The continued fraction's vector-Jacobian product gives abar_k, bbar_k
-//     and E0bar on the host; the recurrence is then reversed step by step
+//     and E0bar; the recurrence is then reversed step by step
 //     (one H*w product and one bilinear <wbar_k|dH|v_k> per step), with the
 //     Lanczos vectors recomputed from checkpoints every m steps (m ~ sqrt(2K)).
 //     The start-vector cotangent goes back through C^T (the same c/c+ map with
@@ -20,7 +20,6 @@
 // All vectors and arithmetic are FP64.
 #include <algorithm>
 #include <cmath>
-#include <complex>
 #include <cstdio>
 #include <cstring>
 #include <memory>
@@ -39,21 +38,65 @@ void edk_internal_add_launches(edk_ctx *ctx, int64_t n);
 int edk_internal_h_sibling(edk_h *h, int nup, int ndn, edk_h **out);
 const uint64_t *edk_internal_h_states(const edk_h *h, int spin);
 int edk_internal_h_is_sz(const edk_h *h);
+const int32_t *edk_internal_h_rank(const edk_h *h);
+cudaMemPool_t edk_internal_pool(edk_ctx *ctx);
 }
 
 using namespace edk;
 
 namespace {
 
+// Device memory from the context's stream-ordered pool (plain memory without one).
 struct DBuf {
     void *p = nullptr;
+    cudaStream_t st = nullptr;
+    bool pooled = false;
     DBuf() = default;
-    explicit DBuf(size_t bytes) { if (cudaMalloc(&p, bytes ? bytes : 16) != cudaSuccess) p = nullptr; }
-    DBuf(DBuf &&o) noexcept : p(o.p) { o.p = nullptr; }
-    DBuf &operator=(DBuf &&o) noexcept { std::swap(p, o.p); return *this; }
+    DBuf(size_t bytes, edk_ctx *ctx) : st(edk_internal_stream(ctx))
+    {
+        if (!bytes) bytes = 16;
+        const cudaMemPool_t pool = edk_internal_pool(ctx);
+        pooled = pool != nullptr;
+        const cudaError_t e = pooled ? cudaMallocFromPoolAsync(&p, bytes, pool, st) : cudaMalloc(&p, bytes);
+        if (e != cudaSuccess) {
+            (void)cudaGetLastError();
+            p = nullptr;
+        }
+    }
+    DBuf(DBuf &&o) noexcept : p(o.p), st(o.st), pooled(o.pooled) { o.p = nullptr; }
+    DBuf &operator=(DBuf &&o) noexcept
+    {
+        std::swap(p, o.p);
+        std::swap(st, o.st);
+        std::swap(pooled, o.pooled);
+        return *this;
+    }
     DBuf(const DBuf &) = delete;
-    ~DBuf() { if (p) cudaFree(p); }
+    ~DBuf()
+    {
+        if (p && pooled) cudaFreeAsync(p, st);
+        else if (p) cudaFree(p);
+    }
     double *d() const { return static_cast<double *>(p); }
+};
+
+// After a call: the pool keeps what it held before it, or up to 1 GB.
+struct PoolGuard {
+    edk_ctx *ctx;
+    cudaMemPool_t pool;
+    uint64_t before = 0;
+    explicit PoolGuard(edk_ctx *c) : ctx(c), pool(edk_internal_pool(c))
+    {
+        if (pool) cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &before);
+    }
+    ~PoolGuard()
+    {
+        uint64_t now = 0;
+        if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &now) != cudaSuccess) return;
+        const uint64_t keep = std::max<uint64_t>(before, (uint64_t)1 << 30);
+        if (now > keep && cudaStreamSynchronize(edk_internal_stream(ctx)) == cudaSuccess)
+            cudaMemPoolTrimTo(pool, (size_t)keep);
+    }
 };
 
 struct HDel {
@@ -77,8 +120,9 @@ struct Ops {
     cudaStream_t st = nullptr;
     int64_t dup = 0, ddn = 0, dim = 0;
     int np = 0, grid = 0;
-    DBuf st_up, st_dn, params, scratch;
-    std::vector<DBuf> maps;
+    DBuf tables, scratch;       // parameters, spin states and hop maps in one upload
+    const uint32_t *st_up = nullptr, *st_dn = nullptr;
+    const ParamDev *params = nullptr;
     double *partials = nullptr, *out = nullptr;
     unsigned *counter = nullptr;
     int fail(int code, const char *msg) { return edk_internal_fail(ctx, code, msg); }
@@ -93,20 +137,14 @@ struct Ops {
 
 // Map of the symmetric hop c+_p c_q + c+_q c_p on one spin's basis:
 // (rank of the target + 1) * sign, 0 where the hop does not apply.
-int hop_map(const uint64_t *states, int64_t n, int p, int q, std::vector<int32_t> &map)
+void hop_map(const uint64_t *states, const int32_t *rank, int64_t n, int p, int q, int32_t *map)
 {
-    map.assign(n, 0);
     const uint64_t bp = 1ull << p, bq = 1ull << q;
     for (int64_t i = 0; i < n; ++i) {
         const uint64_t s = states[i];
         const bool hp = (s & bp) != 0, hq = (s & bq) != 0;
-        if (hp == hq) continue;
-        const uint64_t t = s ^ bp ^ bq;
-        const uint64_t *it = std::lower_bound(states, states + n, t);
-        if (it == states + n || *it != t) return EDK_ERR_INVALID;
-        map[i] = (int32_t)((it - states) + 1) * hop_sign(s, p, q);
+        map[i] = hp == hq ? 0 : (rank[s ^ bp ^ bq] + 1) * hop_sign(s, p, q);
     }
-    return EDK_OK;
 }
 
 int ops_setup(edk_h *h, int np, const edk_param *prm, Ops &o)
@@ -122,17 +160,15 @@ int ops_setup(edk_h *h, int np, const edk_param *prm, Ops &o)
     const int ns = nc + nb;
     if (ns > 32) return o.fail(EDK_ERR_UNSUPPORTED, "gradients need at most 32 orbitals per spin");
     const uint64_t *su = edk_internal_h_states(h, 0), *sd = edk_internal_h_states(h, 1);
-    std::vector<uint32_t> u32(su, su + o.dup), d32(sd, sd + o.ddn);
+    const int32_t *rank = edk_internal_h_rank(h);
     int rc;
-    o.st_up = DBuf(sizeof(uint32_t) * std::max<int64_t>(o.dup, 1));
-    o.st_dn = DBuf(sizeof(uint32_t) * std::max<int64_t>(o.ddn, 1));
-    if (!o.st_up.p || !o.st_dn.p) return o.fail(EDK_ERR_NOMEM, "gradient tables");
-    if ((rc = o.cuda(cudaMemcpy(o.st_up.p, u32.data(), sizeof(uint32_t) * o.dup, cudaMemcpyHostToDevice), "h2d")))
-        return rc;
-    if ((rc = o.cuda(cudaMemcpy(o.st_dn.p, d32.data(), sizeof(uint32_t) * o.ddn, cudaMemcpyHostToDevice), "h2d")))
-        return rc;
+    // words of the upload: the parameters, the spin states, then the maps
+    const size_t pw = sizeof(ParamDev) / 4 * (size_t)np;
+    std::vector<uint32_t> up(pw);
+    up.insert(up.end(), su, su + o.dup);
+    up.insert(up.end(), sd, sd + o.ddn);
     std::vector<ParamDev> pd(np);
-    std::vector<int32_t> map;
+    std::vector<size_t> at[2] = {std::vector<size_t>(np, 0), std::vector<size_t>(np, 0)};
     for (int q = 0; q < np; ++q) {
         const edk_param &p = prm[q];
         ParamDev &d = pd[q];
@@ -167,44 +203,56 @@ int ops_setup(edk_h *h, int np, const edk_param *prm, Ops &o)
             for (int s = 0; s < 2; ++s) {
                 if (!((d.spin_mask >> s) & 1)) continue;
                 const int64_t n = s == 0 ? o.dup : o.ddn;
-                if (hop_map(s == 0 ? su : sd, n, a, b, map)) return o.fail(EDK_ERR_INVALID, "hop map");
-                o.maps.emplace_back(sizeof(int32_t) * std::max<int64_t>(n, 1));
-                if (!o.maps.back().p) return o.fail(EDK_ERR_NOMEM, "gradient maps");
-                if ((rc = o.cuda(cudaMemcpy(o.maps.back().p, map.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice),
-                                 "h2d")))
-                    return rc;
-                (s == 0 ? d.mapu : d.mapd) = static_cast<const int32_t *>(o.maps.back().p);
+                at[s][q] = up.size();
+                up.resize(up.size() + (size_t)n);
+                hop_map(s == 0 ? su : sd, rank, n, a, b, reinterpret_cast<int32_t *>(up.data() + at[s][q]));
             }
         }
     }
-    o.params = DBuf(sizeof(ParamDev) * np);
-    if (!o.params.p) return o.fail(EDK_ERR_NOMEM, "gradient params");
-    if ((rc = o.cuda(cudaMemcpy(o.params.p, pd.data(), sizeof(ParamDev) * np, cudaMemcpyHostToDevice), "h2d")))
+    o.tables = DBuf(sizeof(uint32_t) * up.size(), o.ctx);
+    if (!o.tables.p) return o.fail(EDK_ERR_NOMEM, "gradient tables");
+    const uint32_t *dev_up = static_cast<const uint32_t *>(o.tables.p);
+    for (int q = 0; q < np; ++q) {
+        if (at[0][q]) pd[q].mapu = reinterpret_cast<const int32_t *>(dev_up + at[0][q]);
+        if (at[1][q]) pd[q].mapd = reinterpret_cast<const int32_t *>(dev_up + at[1][q]);
+    }
+    std::memcpy(up.data(), pd.data(), sizeof(ParamDev) * np);
+    o.params = static_cast<const ParamDev *>(o.tables.p);
+    o.st_up = dev_up + pw;
+    o.st_dn = dev_up + pw + o.dup;
+    if ((rc = o.cuda(cudaMemcpyAsync(o.tables.p, up.data(), sizeof(uint32_t) * up.size(), cudaMemcpyHostToDevice, o.st),
+                     "h2d")))
         return rc;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     o.grid = sms * 4;
     const size_t nq = std::max(np, 4);
-    o.scratch = DBuf(sizeof(double) * ((size_t)o.grid * nq + nq + 4) + 64);
+    o.scratch = DBuf(sizeof(double) * ((size_t)o.grid * nq + nq + 4) + 64, o.ctx);
     if (!o.scratch.p) return o.fail(EDK_ERR_NOMEM, "gradient scratch");
     o.partials = o.scratch.d();
     o.out = o.partials + (size_t)o.grid * nq;
     o.counter = reinterpret_cast<unsigned *>(o.out + nq + 2);
-    if ((rc = o.cuda(cudaMemset(o.counter, 0, 16), "memset"))) return rc;
+    if ((rc = o.cuda(cudaMemsetAsync(o.counter, 0, 16, o.st), "memset"))) return rc;
+    // the upload reads the host vector before it goes out of scope
+    if ((rc = o.cuda(cudaStreamSynchronize(o.st), "sync"))) return rc;
     edk_internal_count(o.ctx, (int64_t)(sizeof(uint32_t) * (o.dup + o.ddn) + sizeof(ParamDev) * np), 0);
     return EDK_OK;
 }
 
-// <a|dH_q|b> for every parameter, to the host.
+// <a|dH_q|b> for every parameter, into `out` on the device (added to it when acc).
+int ops_bilinear_dev(Ops &o, const double *a, const double *b, double *out, bool acc)
+{
+    edk_internal_add_launches(o.ctx, 1);
+    return o.cuda(launch_bilinear(o.dup, o.ddn, a, b, o.st_up, o.st_dn, o.np, o.params, o.partials, o.counter, out,
+                                  o.grid, acc, o.st),
+                  "bilinear kernel");
+}
+
+// The same to the host.
 int ops_bilinear(Ops &o, const double *a, const double *b, double *out_host)
 {
-    int rc = o.cuda(launch_bilinear(o.dup, o.ddn, a, b, static_cast<const uint32_t *>(o.st_up.p),
-                                    static_cast<const uint32_t *>(o.st_dn.p), o.np,
-                                    static_cast<const ParamDev *>(o.params.p), o.partials, o.counter, o.out, o.grid,
-                                    o.st),
-                    "bilinear kernel");
-    edk_internal_add_launches(o.ctx, 1);
+    int rc = ops_bilinear_dev(o, a, b, o.out, false);
     if (rc) return rc;
     if ((rc = o.cuda(cudaMemcpyAsync(out_host, o.out, sizeof(double) * o.np, cudaMemcpyDeviceToHost, o.st), "d2h")))
         return rc;
@@ -238,55 +286,13 @@ struct Vec {
     }
 };
 
-// ---- continued-fraction VJP (host) ----------------------------------------
-// G(z) = s u_1 with (z - ph (T - e0)) u = e1, s = b1^2; al[k] (0-based) are the
-// diagonal, be[k] (k = 1..K-1) couples levels k-1 and k.
-void cf_vjp(int K, const double *al, const double *be, double b1, double e0, double ph, int nw, const double *wn,
-            const double *gbar, std::vector<double> &abar, std::vector<double> &bbar, double &b1bar, double &e0bar,
-            double *G_out)
-{
-    using cd = std::complex<double>;
-    abar.assign(K, 0.0);
-    bbar.assign(K + 1, 0.0);
-    b1bar = 0.0;
-    e0bar = 0.0;
-    const double s = b1 * b1;
-    std::vector<cd> d(K), u(K), cp(K), dp(K);
-    for (int w = 0; w < nw; ++w) {
-        const cd z(0.0, wn[w]);
-        // tridiagonal solve (Thomas): diagonal z - ph (a_k - e0), off-diagonal -ph b_k
-        for (int k = 0; k < K; ++k) d[k] = z - ph * (al[k] - e0);
-        cd denom = d[0];
-        cp[0] = K > 1 ? cd(-ph * be[1]) / denom : cd(0.0);
-        dp[0] = cd(1.0) / denom;
-        for (int k = 1; k < K; ++k) {
-            const cd off = -ph * be[k];
-            denom = d[k] - off * cp[k - 1];
-            cp[k] = k + 1 < K ? cd(-ph * be[k + 1]) / denom : cd(0.0);
-            dp[k] = (cd(0.0) - off * dp[k - 1]) / denom;
-        }
-        u[K - 1] = dp[K - 1];
-        for (int k = K - 2; k >= 0; --k) u[k] = dp[k] - cp[k] * u[k + 1];
-        const cd f = u[0];
-        if (G_out) {
-            G_out[2 * w] = (s * f).real();
-            G_out[2 * w + 1] = (s * f).imag();
-        }
-        const cd gc = std::conj(cd(gbar[2 * w], gbar[2 * w + 1]));
-        cd uu(0.0);
-        for (int k = 0; k < K; ++k) {
-            abar[k] += (gc * s * ph * u[k] * u[k]).real();
-            uu += u[k] * u[k];
-            if (k + 1 < K) bbar[k + 1] += (gc * s * 2.0 * ph * u[k] * u[k + 1]).real();
-        }
-        e0bar += (gc * s * (-ph) * uu).real();
-        b1bar += (gc * 2.0 * b1 * f).real();
-    }
-}
-
-// Forward Lanczos of phi (K steps or until breakdown) keeping checkpoints, CF
-// VJP, then the reverse sweep.  Adds to theta_bar (target-sector parameters),
-// writes phibar (target sector) and returns the e0bar of this chain.
+// Forward Lanczos of phi (K steps or until breakdown) keeping checkpoints, the
+// continued fraction with its vector-Jacobian product, then the reverse sweep, all
+// queued on the stream: every coefficient stays on the device (GradScalars), and
+// the host reads b_k once, to learn where the chain ends.  Adds to theta_bar
+// (target-sector parameters), writes phibar (target sector) and returns the e0bar
+// of this chain.
+//   G(z) = b_1^2 u_1 with (z - ph (T - e0)) u = e1.
 int chain_vjp(edk_h *ht, Ops &o, const double *phi, int K, double e0, double ph, int nw, const double *wn,
               const double *gbar, double *theta_bar, double *phibar, double &e0bar_out, double *G_out,
               edk_grad_stats *stats)
@@ -295,7 +301,6 @@ int chain_vjp(edk_h *ht, Ops &o, const double *phi, int K, double e0, double ph,
     const int64_t n = o.dim;
     const size_t vb = sizeof(double) * (size_t)n;
     int rc;
-    // ---- forward ----
     double nrm2 = 0.0;
     if ((rc = v.dots(&nrm2, phi, phi))) return rc;
     const double b1 = std::sqrt(nrm2);
@@ -303,73 +308,78 @@ int chain_vjp(edk_h *ht, Ops &o, const double *phi, int K, double e0, double ph,
     K = (int)std::min<int64_t>(K, n);
     const int m = std::max(2, (int)std::ceil(std::sqrt(2.0 * K)));
     const int nseg = (K + m - 1) / m;
+    // scalars (K + 2 each), theta, and the continued fraction's buffers
+    const size_t ks = (size_t)K + 2, nsc = 4 * ks + 8 + o.np;
+    DBuf sc(sizeof(double) * nsc, o.ctx), cf(sizeof(double) * ((size_t)nw * (4 * (size_t)K + 9)), o.ctx);
+    if (!sc.p || !cf.p) return o.fail(EDK_ERR_NOMEM, "gradient scalars");
+    const GradScalars S{sc.d(), sc.d() + ks, sc.d() + 2 * ks, sc.d() + 3 * ks, sc.d() + 4 * ks};
+    double *theta = sc.d() + 4 * ks + 8;
+    double2 *cf_cp = reinterpret_cast<double2 *>(cf.p), *cf_u = cf_cp + (size_t)K * nw, *cf_gs = cf_u + (size_t)K * nw;
+    double *cf_in = reinterpret_cast<double *>(cf_gs + nw), *cf_G = cf_in + 3 * (size_t)nw, *cf_parts = cf_G + 2 * (size_t)nw;
+    std::vector<double> in(wn, wn + nw);
+    in.insert(in.end(), gbar, gbar + 2 * (size_t)nw);
+    if ((rc = o.cuda(cudaMemsetAsync(sc.p, 0, sizeof(double) * nsc, o.st), "memset"))) return rc;
+    if ((rc = o.cuda(cudaMemcpyAsync(S.be + 1, &b1, sizeof b1, cudaMemcpyHostToDevice, o.st), "h2d"))) return rc;
+    if ((rc = o.cuda(cudaMemcpyAsync(cf_in, in.data(), sizeof(double) * in.size(), cudaMemcpyHostToDevice, o.st), "h2d")))
+        return rc;
+    const GradPass ps{n, o.grid, o.partials, o.counter, o.st};
+    auto count = [&](cudaError_t e, const char *where, int launches = 1) {
+        edk_internal_add_launches(o.ctx, launches);
+        return o.cuda(e, where);
+    };
+    // ---- forward ----
     std::vector<DBuf> ck(2 * nseg);       // (v_{s-1}, v_s) at segment starts s = 1 + j m
-    DBuf va(vb), vbuf(vb), vc(vb), hv(vb);
-    if (!va.p || !vbuf.p || !vc.p || !hv.p) return o.fail(EDK_ERR_NOMEM, "gradient vectors");
-    double *vkm1 = va.d(), *vk = vbuf.d(), *vnext = vc.d();
-    if ((rc = o.cuda(cudaMemsetAsync(vkm1, 0, vb, o.st), "memset"))) return rc;
-    if ((rc = v.lincomb(vk, false, phi, 1.0 / b1))) return rc;
-    std::vector<double> al(K + 1, 0.0), be(K + 2, 0.0);   // al[k-1] = a_k; be[k] = b_k (be[1] = b1)
-    be[1] = b1;
-    int Keff = K;
-    for (int k = 1; k <= K; ++k) {
-        if ((k - 1) % m == 0) {
-            const int j = (k - 1) / m;
-            ck[2 * j] = DBuf(vb);
-            ck[2 * j + 1] = DBuf(vb);
-            if (!ck[2 * j].p || !ck[2 * j + 1].p) return o.fail(EDK_ERR_NOMEM, "gradient checkpoints");
-            if ((rc = o.cuda(cudaMemcpyAsync(ck[2 * j].p, vkm1, vb, cudaMemcpyDeviceToDevice, o.st), "copy"))) return rc;
-            if ((rc = o.cuda(cudaMemcpyAsync(ck[2 * j + 1].p, vk, vb, cudaMemcpyDeviceToDevice, o.st), "copy")))
-                return rc;
+    std::vector<double> be(K + 2, 0.0);
+    {
+        DBuf va(vb, o.ctx), vbuf(vb, o.ctx), vc(vb, o.ctx), hv(vb, o.ctx);
+        if (!va.p || !vbuf.p || !vc.p || !hv.p) return o.fail(EDK_ERR_NOMEM, "gradient vectors");
+        double *vkm1 = va.d(), *vk = vbuf.d(), *vnext = vc.d();
+        if ((rc = o.cuda(cudaMemsetAsync(vkm1, 0, vb, o.st), "memset"))) return rc;
+        if ((rc = v.lincomb(vk, false, phi, 1.0 / b1))) return rc;
+        for (int k = 1; k <= K; ++k) {
+            if ((k - 1) % m == 0) {
+                const int j = (k - 1) / m;
+                ck[2 * j] = DBuf(vb, o.ctx);
+                ck[2 * j + 1] = DBuf(vb, o.ctx);
+                if (!ck[2 * j].p || !ck[2 * j + 1].p) return o.fail(EDK_ERR_NOMEM, "gradient checkpoints");
+                if ((rc = o.cuda(cudaMemcpyAsync(ck[2 * j].p, vkm1, vb, cudaMemcpyDeviceToDevice, o.st), "copy")))
+                    return rc;
+                if ((rc = o.cuda(cudaMemcpyAsync(ck[2 * j + 1].p, vk, vb, cudaMemcpyDeviceToDevice, o.st), "copy")))
+                    return rc;
+            }
+            if ((rc = edk_hmult(ht, EDK_F64, n, vk, hv.p))) return rc;
+            if ((rc = count(pass_fwd_w(ps, hv.d(), vkm1, vk, k, S), "gradient forward"))) return rc;
+            if ((rc = count(pass_fwd_r(ps, vnext, hv.d(), vk, k, S), "gradient forward"))) return rc;
+            if (k == K) break;
+            if ((rc = count(pass_fwd_scale(ps, vnext, k, S), "gradient forward"))) return rc;
+            std::swap(vkm1, vk);
+            std::swap(vk, vnext);
         }
-        if ((rc = edk_hmult(ht, EDK_F64, n, vk, hv.p))) return rc;
-        // w = H v_k - b_k v_{k-1}; a_k = <w, v_k>
-        if ((rc = v.lincomb(hv.d(), true, vkm1, -be[k]))) return rc;
-        double a = 0.0;
-        if ((rc = v.dots(&a, hv.d(), vk))) return rc;
-        al[k - 1] = a;
-        // r = w - a v_k; b_{k+1} = |r|; v_{k+1} = r / b_{k+1}
-        if ((rc = v.lincomb(vnext, false, hv.d(), 1.0, vk, -a))) return rc;
-        double r2 = 0.0;
-        if ((rc = v.dots(&r2, vnext, vnext))) return rc;
-        const double bn = std::sqrt(std::max(r2, 0.0));
-        be[k + 1] = bn;
-        if (stats) stats->forward_steps++;
-        if (!(bn > 1e-25) || k == K) {
-            Keff = k;
-            break;
-        }
-        if ((rc = v.lincomb(vnext, false, vnext, 1.0 / bn))) return rc;
-        std::swap(vkm1, vk);
-        std::swap(vk, vnext);
-    }
+        if ((rc = o.cuda(cudaMemcpyAsync(be.data(), S.be, sizeof(double) * (K + 2), cudaMemcpyDeviceToHost, o.st), "d2h")))
+            return rc;
+        if ((rc = o.cuda(cudaStreamSynchronize(o.st), "sync"))) return rc;
+    }   // the forward vectors are not needed any more
+    int Keff = 1;
+    while (Keff < K && be[Keff + 1] > 1e-25) ++Keff;
+    if (stats) stats->forward_steps += Keff;
     const bool has_next = be[Keff + 1] > 1e-25;
-    va = DBuf();   // the forward vectors are not needed any more
-    vbuf = DBuf();
-    vc = DBuf();
-    hv = DBuf();
     // ---- continued fraction and its VJP ----
-    std::vector<double> abar, bbar;
-    double b1bar = 0.0, e0bar = 0.0;
-    cf_vjp(Keff, al.data(), be.data() + 1, b1, e0, ph, nw, wn, gbar, abar, bbar, b1bar, e0bar, G_out);
-    // bbar[k] of the 0-based helper is the adjoint of b_{k+1} here
-    std::vector<double> bb(Keff + 2, 0.0);
-    for (int k = 1; k < Keff; ++k) bb[k + 1] = bbar[k];
-    bb[1] = b1bar;
+    if ((rc = count(pass_cf(Keff, e0, ph, nw, cf_in, cf_in + nw, S, cf_cp, cf_u, cf_gs, cf_G, cf_parts, o.st),
+                    "gradient continued fraction", 2)))
+        return rc;
     // ---- reverse sweep over segments, last first ----
     const int mseg = m + 2;
     std::vector<DBuf> seg(mseg);
     for (auto &sg : seg) {
-        sg = DBuf(vb);
+        sg = DBuf(vb, o.ctx);
         if (!sg.p) return o.fail(EDK_ERR_NOMEM, "gradient segment");
     }
     if (stats) stats->stored_vectors = std::max<int32_t>(stats->stored_vectors, 2 * nseg + mseg + 4);
-    DBuf vbn_b(vb), vbc_b(vb), wbar_b(vb), rbar_b(vb);
-    if (!vbn_b.p || !vbc_b.p || !wbar_b.p || !rbar_b.p) return o.fail(EDK_ERR_NOMEM, "gradient adjoints");
-    double *vbn = vbn_b.d(), *vbc = vbc_b.d(), *wbar = wbar_b.d(), *rbar = rbar_b.d();
+    DBuf vbn_b(vb, o.ctx), vbc_b(vb, o.ctx), wbar_b(vb, o.ctx), hw_b(vb, o.ctx);
+    if (!vbn_b.p || !vbc_b.p || !wbar_b.p || !hw_b.p) return o.fail(EDK_ERR_NOMEM, "gradient adjoints");
+    double *vbn = vbn_b.d(), *vbc = vbc_b.d(), *wbar = wbar_b.d();
     if ((rc = o.cuda(cudaMemsetAsync(vbn, 0, vb, o.st), "memset"))) return rc;   // vbar_{Keff+1} = 0
     if ((rc = o.cuda(cudaMemsetAsync(vbc, 0, vb, o.st), "memset"))) return rc;   // vbar_{Keff} (partial)
-    std::vector<double> tb(o.np);
     const int jlast = (Keff - 1) / m;
     for (int j = jlast; j >= 0; --j) {
         const int s0 = 1 + j * m, e1 = std::min(s0 + m - 1, Keff);
@@ -385,57 +395,34 @@ int chain_vjp(edk_h *ht, Ops &o, const double *phi, int K, double e0, double ph,
                 continue;
             }
             if ((rc = edk_hmult(ht, EDK_F64, n, seg[i].p, seg[i + 1].p))) return rc;
-            if ((rc = v.lincomb(seg[i + 1].d(), true, seg[i - 1].d(), -be[k], seg[i].d(), -al[k - 1]))) return rc;
-            if ((rc = v.lincomb(seg[i + 1].d(), false, seg[i + 1].d(), 1.0 / be[k + 1]))) return rc;
+            if ((rc = count(pass_replay(ps, seg[i + 1].d(), seg[i - 1].d(), seg[i].d(), k, S), "gradient replay")))
+                return rc;
             if (stats) stats->replay_steps++;
         }
         for (int k = e1; k >= s0; --k) {
             const int i = k - (s0 - 1);
             const double *vkp = seg[i + 1].d(), *vkk = seg[i].d(), *vkm = seg[i - 1].d();
-            const double ak = al[k - 1], bk = be[k], bk1 = be[k + 1];
-            bool have_r = false;
-            if (k < Keff) {
-                // rbar = vbar_{k+1} / b_{k+1} + (bb_{k+1} - <vbar_{k+1}, v_{k+1}> / b_{k+1}) v_{k+1}
-                double d1 = 0.0;
-                if ((rc = v.dots(&d1, vbn, vkp))) return rc;
-                if ((rc = v.lincomb(rbar, false, vbn, 1.0 / bk1, vkp, bb[k + 1] - d1 / bk1))) return rc;
-                have_r = true;
-            }
-            // abar' = abar_k - <rbar, v_k>; wbar = rbar + abar' v_k
-            double d2 = 0.0;
-            if (have_r && (rc = v.dots(&d2, rbar, vkk))) return rc;
-            const double ab = abar[k - 1] - d2;
-            if (have_r) {
-                if ((rc = v.lincomb(wbar, false, rbar, 1.0, vkk, ab))) return rc;
-                // vbar_k += -a_k rbar + abar' w_k,  w_k = b_{k+1} v_{k+1} + a_k v_k
-                if ((rc = v.lincomb(vbc, true, rbar, -ak, vkp, ab * bk1, vkk, ab * ak))) return rc;
-            } else {
-                if ((rc = v.lincomb(wbar, false, vkk, ab))) return rc;
-                if ((rc = v.lincomb(vbc, true, vkp, ab * bk1, vkk, ab * ak))) return rc;
-            }
-            // vbar_k += H wbar
-            if ((rc = edk_hmult(ht, EDK_F64, n, wbar, rbar))) return rc;
-            if ((rc = v.lincomb(vbc, true, rbar, 1.0))) return rc;
+            if ((rc = count(pass_rev_wbar(ps, k < Keff, vbn, vbc, wbar, vkp, vkk, vkm, k, S), "gradient reverse")))
+                return rc;
+            if ((rc = edk_hmult(ht, EDK_F64, n, wbar, hw_b.p))) return rc;
             // theta_bar += <wbar| dH |v_k>
-            if ((rc = ops_bilinear(o, wbar, vkk, tb.data()))) return rc;
-            for (int q = 0; q < o.np; ++q) theta_bar[q] += tb[q];
-            // bb_k -= <wbar, v_{k-1}>; vbar_{k-1} starts at -b_k wbar
-            if (k >= 2) {
-                double d3 = 0.0;
-                if ((rc = v.dots(&d3, wbar, vkm))) return rc;
-                bb[k] -= d3;
-            }
+            if ((rc = ops_bilinear_dev(o, wbar, vkk, theta, true))) return rc;
+            if ((rc = count(pass_rev_next(ps, vbn, vbc, hw_b.d(), wbar, vkk, vkm, k, S), "gradient reverse"))) return rc;
             std::swap(vbn, vbc);
-            if ((rc = v.lincomb(vbc, false, wbar, -bk))) return rc;
             if (stats) stats->reverse_steps++;
         }
     }
-    // vbn = vbar_1; seg[1] = v_1 (replay of the first segment).  v_1 = phi / b1, b1 = |phi|:
-    // phibar = (vbar_1 - <vbar_1, v_1> v_1) / b1 + bb_1 v_1
-    double d4 = 0.0;
-    if ((rc = v.dots(&d4, vbn, seg[1].d()))) return rc;
-    if ((rc = v.lincomb(phibar, false, vbn, 1.0 / b1, seg[1].d(), -d4 / b1 + bb[1]))) return rc;
-    e0bar_out = e0bar;
+    // vbn = vbar_1; seg[1] = v_1 (replay of the first segment)
+    if ((rc = count(pass_rev_start(ps, phibar, vbn, seg[1].d(), S), "gradient reverse"))) return rc;
+    std::vector<double> th(o.np);
+    if ((rc = o.cuda(cudaMemcpyAsync(th.data(), theta, sizeof(double) * o.np, cudaMemcpyDeviceToHost, o.st), "d2h")))
+        return rc;
+    if ((rc = o.cuda(cudaMemcpyAsync(&e0bar_out, S.dot + 4, sizeof(double), cudaMemcpyDeviceToHost, o.st), "d2h")))
+        return rc;
+    if (G_out && (rc = o.cuda(cudaMemcpyAsync(G_out, cf_G, sizeof(double) * 2 * nw, cudaMemcpyDeviceToHost, o.st), "d2h")))
+        return rc;
+    if ((rc = o.cuda(cudaStreamSynchronize(o.st), "sync"))) return rc;
+    for (int q = 0; q < o.np; ++q) theta_bar[q] += th[q];
     return EDK_OK;
 }
 
@@ -478,6 +465,7 @@ int edk_grad_green(edk_h *h, const void *psi_dev, double e0, int32_t nchain, con
         (nchain > 0 && (nw < 1 || nitergreen < 1)))
         return EDK_ERR_INVALID;
     if (stats) std::memset(stats, 0, sizeof *stats);
+    PoolGuard guard(edk_internal_h_ctx(h));
     Ops o;
     int rc = ops_setup(h, np, params, o);
     if (rc) return rc;
@@ -488,7 +476,7 @@ int edk_grad_green(edk_h *h, const void *psi_dev, double e0, int32_t nchain, con
     edk_internal_h_info(h, &nc, &nb, &nup, &ndn);
     const int ns = nc + nb;
     // normalised psi
-    DBuf psi_b(vb), psibar_b(vb);
+    DBuf psi_b(vb, o.ctx), psibar_b(vb, o.ctx);
     if (!psi_b.p || !psibar_b.p) return o.fail(EDK_ERR_NOMEM, "gradient vectors");
     double n2 = 0.0;
     if ((rc = v.dots(&n2, static_cast<const double *>(psi_dev), static_cast<const double *>(psi_dev)))) return rc;
@@ -514,7 +502,7 @@ int edk_grad_green(edk_h *h, const void *psi_dev, double e0, int32_t nchain, con
         Ops ot;
         if ((rc = ops_setup(ht.get(), np, params, ot))) return rc;
         const size_t tvb = sizeof(double) * (size_t)ot.dim;
-        DBuf phi(tvb), phibar(tvb);
+        DBuf phi(tvb, o.ctx), phibar(tvb, o.ctx);
         if (!phi.p || !phibar.p) return o.fail(EDK_ERR_NOMEM, "gradient vectors");
         int64_t od = 0;
         if ((rc = edk_apply_c(h, EDK_F64, g.site, g.spin, g.dagger ? 1 : 0, g.site2, g.sign2, psi, phi.p, &od)))
@@ -528,7 +516,7 @@ int edk_grad_green(edk_h *h, const void *psi_dev, double e0, int32_t nchain, con
         for (int q = 0; q < np; ++q) grad[q] += tg[q];
         e0bar_total += e0b;
         // psibar += C^T phibar (the map with dagger flipped, from the target sector back)
-        DBuf back(vb);
+        DBuf back(vb, o.ctx);
         if (!back.p) return o.fail(EDK_ERR_NOMEM, "gradient vectors");
         if ((rc = edk_apply_c(ht.get(), EDK_F64, g.site, g.spin, g.dagger ? 0 : 1, g.site2, g.sign2, phibar.p, back.p,
                               &od)))
@@ -543,39 +531,34 @@ int edk_grad_green(edk_h *h, const void *psi_dev, double e0, int32_t nchain, con
         double pp[2];
         if ((rc = v.dots(pp, psibar_b.d(), psi, psibar_b.d(), psibar_b.d()))) return rc;
         if (pp[1] > 0.0) {
-            DBuf x_b(vb), r_b(vb), p_b(vb), ap_b(vb);
-            if (!x_b.p || !r_b.p || !p_b.p || !ap_b.p) return o.fail(EDK_ERR_NOMEM, "gradient CG vectors");
+            DBuf x_b(vb, o.ctx), r_b(vb, o.ctx), p_b(vb, o.ctx), ap_b(vb, o.ctx), cg_b(sizeof(CgScalars), o.ctx);
+            if (!x_b.p || !r_b.p || !p_b.p || !ap_b.p || !cg_b.p) return o.fail(EDK_ERR_NOMEM, "gradient CG vectors");
             double *x = x_b.d(), *r = r_b.d(), *p = p_b.d(), *ap = ap_b.d();
             if ((rc = o.cuda(cudaMemsetAsync(x, 0, vb, o.st), "memset"))) return rc;
             if ((rc = v.lincomb(r, false, psibar_b.d(), 1.0, psi, -pp[0]))) return rc;
             if ((rc = v.lincomb(p, false, r, 1.0))) return rc;
             double rr = 0.0;
             if ((rc = v.dots(&rr, r, r))) return rc;
-            const double rr0 = rr;
             const double tol = cg_tol > 0.0 ? cg_tol : 1e-10;
-            int it = 0;
             const int maxit = 20000;
-            while (rr > tol * tol * rr0 && it < maxit) {
-                if ((rc = edk_hmult(h, EDK_F64, n, p, ap))) return rc;
-                // ap = (H - E0) p, projected off psi
-                double t[2];
-                if ((rc = v.dots(t, ap, psi, p, psi))) return rc;
-                if ((rc = v.lincomb(ap, false, ap, 1.0, p, -e0, psi, -(t[0] - e0 * t[1])))) return rc;
-                double pap = 0.0;
-                if ((rc = v.dots(&pap, p, ap))) return rc;
-                if (!(pap > 0.0)) break;
-                const double alpha = rr / pap;
-                if ((rc = v.lincomb(x, true, p, alpha))) return rc;
-                if ((rc = v.lincomb(r, true, ap, -alpha))) return rc;
-                double rn = 0.0;
-                if ((rc = v.dots(&rn, r, r))) return rc;
-                if ((rc = v.lincomb(p, false, r, 1.0, p, rn / rr))) return rc;
-                rr = rn;
-                ++it;
+            CgScalars cg{rr, rr, {0.0, 0.0}, 0.0, 0.0, 0, rr > tol * tol * rr ? 0 : 1};
+            CgScalars *cgd = static_cast<CgScalars *>(cg_b.p);
+            if ((rc = o.cuda(cudaMemcpyAsync(cgd, &cg, sizeof cg, cudaMemcpyHostToDevice, o.st), "h2d"))) return rc;
+            const GradPass ps{n, o.grid, o.partials, o.counter, o.st};
+            // sixteen iterations are queued between looks at the device's stop flag, which
+            // turns the passes behind the last iteration into no-ops
+            while (!cg.done) {
+                for (int q = 0; q < 16; ++q) {
+                    if ((rc = edk_hmult(h, EDK_F64, n, p, ap))) return rc;
+                    edk_internal_add_launches(o.ctx, 4);
+                    if ((rc = o.cuda(pass_cg(ps, x, r, p, ap, psi, e0, tol * tol, maxit, cgd), "gradient CG"))) return rc;
+                }
+                if ((rc = o.cuda(cudaMemcpyAsync(&cg, cgd, sizeof cg, cudaMemcpyDeviceToHost, o.st), "d2h"))) return rc;
+                if ((rc = o.cuda(cudaStreamSynchronize(o.st), "sync"))) return rc;
             }
             if (stats) {
-                stats->cg_iterations = it;
-                stats->cg_residual = std::sqrt(rr / rr0);
+                stats->cg_iterations = cg.it;
+                stats->cg_residual = std::sqrt(cg.rr / cg.rr0);
             }
             if ((rc = ops_bilinear(o, x, psi, tb.data()))) return rc;
             for (int q = 0; q < np; ++q) grad[q] -= tb[q];

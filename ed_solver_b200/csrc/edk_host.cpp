@@ -1086,6 +1086,11 @@ int edk_internal_h_sibling(edk_h *h, int nup, int ndn, edk_h **out)
 // The basis states of one spin species of the sector (increasing order).
 const uint64_t *edk_internal_h_states(const edk_h *h, int spin) { return h->tab[spin].states.data(); }
 
+const int32_t *edk_internal_h_rank(const edk_h *h) { return h->rank.data(); }
+
+// The context's stream-ordered pool (null when the device has none).
+cudaMemPool_t edk_internal_pool(edk_ctx *ctx) { return ctx->get_basis_pool(); }
+
 int edk_ctx_set_graphs(edk_ctx *ctx, int enable)
 {
     if (!ctx) return EDK_ERR_INVALID;
