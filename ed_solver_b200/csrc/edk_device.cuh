@@ -4,6 +4,7 @@
 #include <cstdint>
 #include <cstring>
 #include "edk_internal.h"
+#include "edk_launch.cuh"
 
 namespace edk {
 

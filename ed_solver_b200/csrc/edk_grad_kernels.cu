@@ -62,12 +62,14 @@ __global__ void __launch_bounds__(512, 1) bilinear_kernel(int dup, int ddn, cons
     __shared__ ParamDev sp[kMaxGradParams];
     __shared__ double s_part[kMaxGradParams][16];
     __shared__ bool last;
+    chain_next();
     const int nwarp = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int share = nwarp > np ? nwarp / np : 1;              // warps per parameter
     const int sub = warp % share, first = warp / share, step = nwarp / share;
     const int c0 = lane + 32 * sub, cs = 32 * share;
     for (int q = threadIdx.x; q < np; q += blockDim.x) sp[q] = P[q];
     for (int t = threadIdx.x; t < np * 16; t += blockDim.x) s_part[t / 16][t % 16] = 0.0;
+    chain_wait();
     double *as = reinterpret_cast<double *>(smem_raw);
     double *bs = as + dup;
     for (int row = blockIdx.x; row < ddn; row += gridDim.x) {
@@ -162,6 +164,8 @@ __global__ void __launch_bounds__(512, 1) bilinear_kernel(int dup, int ddn, cons
 __global__ void fwd_w_kernel(int64_t n, double *w, const double *vkm1, const double *vk, int k, GradScalars S,
                              double *partials, unsigned *counter)
 {
+    chain_next();
+    chain_wait();
     double s[1] = {0.0};
     const double b = -S.be[k];
     EDK_EACH(i) {
@@ -176,6 +180,8 @@ __global__ void fwd_w_kernel(int64_t n, double *w, const double *vkm1, const dou
 __global__ void fwd_r_kernel(int64_t n, double *r, const double *w, const double *vk, int k, GradScalars S,
                              double *partials, unsigned *counter)
 {
+    chain_next();
+    chain_wait();
     double s[1] = {0.0};
     const double a = -S.al[k];
     EDK_EACH(i) {
@@ -189,6 +195,8 @@ __global__ void fwd_r_kernel(int64_t n, double *r, const double *w, const double
 // v_{k+1} = r / b_{k+1} (zero after a breakdown: the host cuts the chain there)
 __global__ void fwd_scale_kernel(int64_t n, double *r, int k, GradScalars S)
 {
+    chain_next();
+    chain_wait();
     const double b = S.be[k + 1], c = b > 1e-25 ? 1.0 / b : 0.0;
     EDK_EACH(i) r[i] = c * r[i];
 }
@@ -196,6 +204,8 @@ __global__ void fwd_scale_kernel(int64_t n, double *r, int k, GradScalars S)
 // v_{k+1} = (H v_k - b_k v_{k-1} - a_k v_k) / b_{k+1}, in place over H v_k
 __global__ void replay_kernel(int64_t n, double *v, const double *vkm1, const double *vk, int k, GradScalars S)
 {
+    chain_next();
+    chain_wait();
     const double b = -S.be[k], a = -S.al[k], c = 1.0 / S.be[k + 1];
     EDK_EACH(i) {
         double t = v[i] + b * vkm1[i];
@@ -213,6 +223,8 @@ __global__ void rev_wbar_kernel(int64_t n, int have_r, const double *vbn, double
                                 const double *vkk, const double *vkm, int k, GradScalars S, double *partials,
                                 unsigned *counter)
 {
+    chain_next();
+    chain_wait();
     const double ak = S.al[k], bk1 = S.be[k + 1];
     double cr = 0.0, ib = 0.0, ab = S.ab[k];
     if (have_r) {
@@ -241,6 +253,8 @@ __global__ void rev_next_kernel(int64_t n, double *vbn, double *vbc, const doubl
                                 const double *vkk, const double *vkm, int k, GradScalars S, double *partials,
                                 unsigned *counter)
 {
+    chain_next();
+    chain_wait();
     const double b = -S.be[k];
     double s[3] = {0.0, 0.0, 0.0};
     EDK_EACH(i) {
@@ -257,6 +271,8 @@ __global__ void rev_next_kernel(int64_t n, double *vbn, double *vbc, const doubl
 // phibar = (vbar_1 - <vbar_1, v_1> v_1) / b_1 + bb_1 v_1
 __global__ void rev_start_kernel(int64_t n, double *phibar, const double *vb1, const double *v1, GradScalars S)
 {
+    chain_next();
+    chain_wait();
     const double b1 = S.be[1], c = -S.dot[0] / b1 + S.bb[1], ib = 1.0 / b1;
     EDK_EACH(i) phibar[i] = ib * vb1[i] + c * v1[i];
 }
@@ -266,6 +282,8 @@ __global__ void rev_start_kernel(int64_t n, double *phibar, const double *vb1, c
 __global__ void cg_dots_kernel(int64_t n, const double *ap, const double *p, const double *psi, CgScalars *S,
                                double *partials, unsigned *counter)
 {
+    chain_next();
+    chain_wait();
     if (S->done) return;
     double s[2] = {0.0, 0.0};
     EDK_EACH(i) {
@@ -277,6 +295,8 @@ __global__ void cg_dots_kernel(int64_t n, const double *ap, const double *p, con
 __global__ void cg_project_kernel(int64_t n, double *ap, const double *p, const double *psi, double e0, CgScalars *S,
                                   double *partials, unsigned *counter)
 {
+    chain_next();
+    chain_wait();
     if (S->done) return;
     const double c = -(S->t[0] - e0 * S->t[1]);
     double s[1] = {0.0};
@@ -291,6 +311,8 @@ __global__ void cg_project_kernel(int64_t n, double *ap, const double *p, const 
 __global__ void cg_step_kernel(int64_t n, double *x, double *r, const double *p, const double *ap, CgScalars *S,
                                double *partials, unsigned *counter)
 {
+    chain_next();
+    chain_wait();
     if (S->done) return;
     const double al = S->rr / S->pap;
     double s[1] = {0.0};
@@ -305,6 +327,8 @@ __global__ void cg_step_kernel(int64_t n, double *x, double *r, const double *p,
 __global__ void cg_direction_kernel(int64_t n, double *p, const double *r, double tol2, int maxit, CgScalars *S,
                                     double *partials, unsigned *counter)
 {
+    chain_next();
+    chain_wait();
     if (S->done) return;
     const double c = S->rn / S->rr;
     EDK_EACH(i) p[i] = r[i] + c * p[i];
@@ -445,16 +469,14 @@ cudaError_t launch_bilinear(int64_t dup, int64_t ddn, const double *a, const dou
     const size_t smem = 2 * (size_t)dup * sizeof(double);
     // the kernel's static shared memory is about 11 KB of the 227 KB a block may use
     if (smem <= (size_t)(227 - 12) * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(bilinear_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
+        int per_sm = 0;
+        cudaError_t e = kernel_fit(reinterpret_cast<const void *>(bilinear_kernel<true>), 512, smem, &per_sm);
         if (e != cudaSuccess) return e;
-        bilinear_kernel<true><<<grid, 512, smem, st>>>((int)dup, (int)ddn, a, b, st_up, st_dn, np, P, partials,
-                                                       counter, out, accumulate ? 1 : 0);
-    } else {
-        bilinear_kernel<false><<<grid, 512, 0, st>>>((int)dup, (int)ddn, a, b, st_up, st_dn, np, P, partials,
-                                                     counter, out, accumulate ? 1 : 0);
+        return launch_chained(bilinear_kernel<true>, grid, 512, smem, st, (int)dup, (int)ddn, a, b, st_up, st_dn, np, P,
+                              partials, counter, out, accumulate ? 1 : 0);
     }
-    return cudaGetLastError();
+    return launch_chained(bilinear_kernel<false>, grid, 512, 0, st, (int)dup, (int)ddn, a, b, st_up, st_dn, np, P,
+                          partials, counter, out, accumulate ? 1 : 0);
 }
 
 // ---- passes of the adjoint (GradPass: sector length, grid, reduction scratch, stream) ----
@@ -465,51 +487,45 @@ static int pass_grid(const GradPass &p)
 }
 cudaError_t pass_fwd_w(const GradPass &p, double *w, const double *vkm1, const double *vk, int k, const GradScalars &S)
 {
-    fwd_w_kernel<<<pass_grid(p), 256, 0, p.st>>>(p.n, w, vkm1, vk, k, S, p.partials, p.counter);
-    return cudaGetLastError();
+    return launch_chained(fwd_w_kernel, pass_grid(p), 256, 0, p.st, p.n, w, vkm1, vk, k, S, p.partials, p.counter);
 }
 cudaError_t pass_fwd_r(const GradPass &p, double *r, const double *w, const double *vk, int k, const GradScalars &S)
 {
-    fwd_r_kernel<<<pass_grid(p), 256, 0, p.st>>>(p.n, r, w, vk, k, S, p.partials, p.counter);
-    return cudaGetLastError();
+    return launch_chained(fwd_r_kernel, pass_grid(p), 256, 0, p.st, p.n, r, w, vk, k, S, p.partials, p.counter);
 }
 cudaError_t pass_fwd_scale(const GradPass &p, double *r, int k, const GradScalars &S)
 {
-    fwd_scale_kernel<<<pass_grid(p), 256, 0, p.st>>>(p.n, r, k, S);
-    return cudaGetLastError();
+    return launch_chained(fwd_scale_kernel, pass_grid(p), 256, 0, p.st, p.n, r, k, S);
 }
 cudaError_t pass_replay(const GradPass &p, double *v, const double *vkm1, const double *vk, int k, const GradScalars &S)
 {
-    replay_kernel<<<pass_grid(p), 256, 0, p.st>>>(p.n, v, vkm1, vk, k, S);
-    return cudaGetLastError();
+    return launch_chained(replay_kernel, pass_grid(p), 256, 0, p.st, p.n, v, vkm1, vk, k, S);
 }
 cudaError_t pass_rev_wbar(const GradPass &p, bool have_r, const double *vbn, double *vbc, double *wbar,
                           const double *vkp, const double *vkk, const double *vkm, int k, const GradScalars &S)
 {
-    rev_wbar_kernel<<<pass_grid(p), 256, 0, p.st>>>(p.n, have_r ? 1 : 0, vbn, vbc, wbar, vkp, vkk, vkm, k, S, p.partials,
+    return launch_chained(rev_wbar_kernel, pass_grid(p), 256, 0, p.st, p.n, have_r ? 1 : 0, vbn, vbc, wbar, vkp, vkk, vkm, k, S, p.partials,
                                                     p.counter);
-    return cudaGetLastError();
 }
 cudaError_t pass_rev_next(const GradPass &p, double *vbn, double *vbc, const double *hw, const double *wbar,
                           const double *vkk, const double *vkm, int k, const GradScalars &S)
 {
-    rev_next_kernel<<<pass_grid(p), 256, 0, p.st>>>(p.n, vbn, vbc, hw, wbar, vkk, vkm, k, S, p.partials, p.counter);
-    return cudaGetLastError();
+    return launch_chained(rev_next_kernel, pass_grid(p), 256, 0, p.st, p.n, vbn, vbc, hw, wbar, vkk, vkm, k, S, p.partials, p.counter);
 }
 cudaError_t pass_rev_start(const GradPass &p, double *phibar, const double *vb1, const double *v1, const GradScalars &S)
 {
-    rev_start_kernel<<<pass_grid(p), 256, 0, p.st>>>(p.n, phibar, vb1, v1, S);
-    return cudaGetLastError();
+    return launch_chained(rev_start_kernel, pass_grid(p), 256, 0, p.st, p.n, phibar, vb1, v1, S);
 }
 cudaError_t pass_cg(const GradPass &p, double *x, double *r, double *d, double *ap, const double *psi, double e0,
                     double tol2, int maxit, CgScalars *S)
 {
     const int g = pass_grid(p);
-    cg_dots_kernel<<<g, 256, 0, p.st>>>(p.n, ap, d, psi, S, p.partials, p.counter);
-    cg_project_kernel<<<g, 256, 0, p.st>>>(p.n, ap, d, psi, e0, S, p.partials, p.counter);
-    cg_step_kernel<<<g, 256, 0, p.st>>>(p.n, x, r, d, ap, S, p.partials, p.counter);
-    cg_direction_kernel<<<g, 256, 0, p.st>>>(p.n, d, r, tol2, maxit, S, p.partials, p.counter);
-    return cudaGetLastError();
+    cudaError_t e = cudaSuccess;
+    if (e == cudaSuccess) e = launch_chained(cg_dots_kernel, g, 256, 0, p.st, p.n, ap, d, psi, S, p.partials, p.counter);
+    if (e == cudaSuccess) e = launch_chained(cg_project_kernel, g, 256, 0, p.st, p.n, ap, d, psi, e0, S, p.partials, p.counter);
+    if (e == cudaSuccess) e = launch_chained(cg_step_kernel, g, 256, 0, p.st, p.n, x, r, d, ap, S, p.partials, p.counter);
+    if (e == cudaSuccess) e = launch_chained(cg_direction_kernel, g, 256, 0, p.st, p.n, d, r, tol2, maxit, S, p.partials, p.counter);
+    return e;
 }
 cudaError_t pass_cf(int K, double e0, double ph, int nw, const double *wn, const double *gbar, const GradScalars &S,
                     double2 *cp, double2 *u, double2 *gs, double *G, double *parts, cudaStream_t st)

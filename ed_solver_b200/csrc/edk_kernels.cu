@@ -35,6 +35,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <cstring>
+#include <vector>
 #include "edk_internal.h"
 #include "edk_device.cuh"
 
@@ -114,6 +115,11 @@ __global__ void __launch_bounds__(512, 1) row_kernel(const HamDev H, const RowAr
     const int64_t dup = H.dup, ddn = H.ddn;
     const T *__restrict__ x = static_cast<const T *>(a.x);
 
+    chain_next();
+    if (PACKED) {
+        for (int i = threadIdx.x; i < H.up.npal; i += blockDim.x) pal_s[i] = H.up.pal[i];
+    }
+    chain_wait();
     // step scalars: s = w_k - gamma_k v_k was stored by the previous launch;
     // delta_k = alpha_k - gamma_k; the new vector is s' = w_{k+1} - gamma_{k+1} v_{k+1}
     // with gamma_{k+1} = alpha_k
@@ -130,9 +136,6 @@ __global__ void __launch_bounds__(512, 1) row_kernel(const HamDev H, const RowAr
         beta_k = ks >= 2 ? a.tri_sub[ks - 1] : 0.0;
         inv_b = 1.0 / beta_k1;
         if (a.psi_coef) cpsi = a.psi_coef[ks];
-    }
-    if (PACKED) {
-        for (int i = threadIdx.x; i < H.up.npal; i += blockDim.x) pal_s[i] = H.up.pal[i];
     }
 
     const uint32_t *__restrict__ ell = H.up.ell;
@@ -474,6 +477,32 @@ __global__ void docc_kernel(int64_t dup, int64_t ddn, const uint8_t *imp_up, con
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
+cudaError_t kernel_fit(const void *kernel, int threads, size_t smem, int *per_sm)
+{
+    struct Fit { const void *kernel; int device, threads; size_t smem; int per_sm; };
+    static thread_local std::vector<Fit> known;      // one entry per kernel and launch shape used
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    for (const Fit &f : known)
+        if (f.kernel == kernel && f.threads == threads && f.smem == smem && f.device == device) {
+            *per_sm = f.per_sm;
+            return cudaSuccess;
+        }
+    // the limit is set to all the kernel can have, so that it holds for every entry
+    cudaFuncAttributes at;
+    int most = 0;
+    if ((e = cudaFuncGetAttributes(&at, kernel)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device)) != cudaSuccess) return e;
+    if (at.sharedSizeBytes + smem > (size_t)most) return cudaErrorInvalidValue;
+    if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  most - (int)at.sharedSizeBytes)) != cudaSuccess)
+        return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, threads, smem)) != cudaSuccess) return e;
+    known.push_back({kernel, device, threads, smem, *per_sm});
+    return cudaSuccess;
+}
+
 LaunchCfg plan_rows(const HamDev &H, int elem_bytes, int num_sms)
 {
     LaunchCfg c;
@@ -526,22 +555,16 @@ template <typename T, int R, bool S, bool P, int KM>
 static cudaError_t launch_rows_k(const HamDev &H, const RowArgs &a, const LaunchCfg &cfg, cudaStream_t st)
 {
     auto k = row_kernel<T, R, S, P, KM>;
-    if (cfg.smem > 0) {
-        // static + dynamic shared memory may exceed the 48 KB default
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.smem);
-        if (e != cudaSuccess) return e;
-    }
     // grid = resident blocks (registers and shared memory of this instance)
     int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, cfg.block, cfg.smem);
+    cudaError_t e = kernel_fit(reinterpret_cast<const void *>(k), cfg.block, cfg.smem, &per_sm);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
     int64_t grid = (int64_t)cfg.num_sms * per_sm;
     if (grid > cfg.groups) grid = cfg.groups;
     if (grid > cfg.grid) grid = cfg.grid;
     if (grid < 1) grid = 1;
-    k<<<(int)grid, cfg.block, cfg.smem, st>>>(H, a);
-    return cudaGetLastError();
+    return launch_chained(k, (int)grid, cfg.block, cfg.smem, st, H, a);
 }
 
 template <typename T, int R, bool S>

@@ -72,6 +72,15 @@ __global__ void __launch_bounds__(NTHR, MINB) row_fast_kernel(const HamDev H, co
     const int64_t ddn = H.ddn;
     const T *__restrict__ x = static_cast<const T *>(a.x);
 
+    chain_next();
+    {
+        for (int i = threadIdx.x; i < H.up.npal; i += blockDim.x) pal_s[i] = H.up.pal[i];
+        const int nio = H.ncfg * H.ncfg + 1;
+        for (int i = threadIdx.x; i < nio; i += blockDim.x) s_ioff[i] = H.int_off[i];
+        const int ncoef = H.int_off[nio - 1];
+        for (int i = threadIdx.x; i < ncoef; i += blockDim.x) s_icoef[i] = H.int_coef[i];
+    }
+    chain_wait();
     // step scalars: s = w_k - gamma_k v_k was stored by the previous launch;
     // delta_k = alpha_k - gamma_k; the new vector is s' = w_{k+1} - gamma_{k+1} v_{k+1}
     // with gamma_{k+1} = alpha_k
@@ -88,13 +97,6 @@ __global__ void __launch_bounds__(NTHR, MINB) row_fast_kernel(const HamDev H, co
         beta_k = ks >= 2 ? a.tri_sub[ks - 1] : 0.0;
         inv_b = 1.0 / beta_k1;
         if (a.psi_coef) cpsi = a.psi_coef[ks];
-    }
-    {
-        for (int i = threadIdx.x; i < H.up.npal; i += blockDim.x) pal_s[i] = H.up.pal[i];
-        const int nio = H.ncfg * H.ncfg + 1;
-        for (int i = threadIdx.x; i < nio; i += blockDim.x) s_ioff[i] = H.int_off[i];
-        const int ncoef = H.int_off[nio - 1];
-        for (int i = threadIdx.x; i < ncoef; i += blockDim.x) s_icoef[i] = H.int_coef[i];
     }
     const uint64_t keep = l2_keep(), stream = l2_stream();
     const uint32_t *__restrict__ ell = H.up.ell;
@@ -303,23 +305,19 @@ cudaError_t launch_fast_t(const HamDev &H, const RowArgs &a, int num_sms, cudaSt
 {
     auto k = row_fast_kernel<T, R, KMU, KMD, NTHR, MINB, CPT>;
     const size_t smem = (size_t)R * (size_t)H.dup * sizeof(T);
-    // static + dynamic shared memory may exceed the 48 KB default
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
     const int cols = (int)((H.dup + CPT - 1) / CPT);
     int block = NTHR;
     if (cols < block) block = ((cols + 31) / 32) * 32;
     if (block < 32) block = 32;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, block, smem);
+    cudaError_t e = kernel_fit(reinterpret_cast<const void *>(k), block, smem, &per_sm);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
     const int64_t groups = (H.ddn + R - 1) / R;
     int64_t grid = (int64_t)num_sms * per_sm;
     if (grid > groups) grid = groups;
     if (grid < 1) grid = 1;
-    k<<<(int)grid, block, smem, st>>>(H, a);
-    return cudaGetLastError();
+    return launch_chained(k, (int)grid, block, smem, st, H, a);
 }
 
 // Shape dispatch for one element type (edk_rows_fast.cu: FP32, edk_rows_fast64.cu: FP64).

@@ -125,21 +125,7 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
     const T *__restrict__ x = static_cast<const T *>(a.x);
     const int tid = threadIdx.x;
 
-    const int mode = STEP ? (int)kModeStep : a.mode;
-    double delta = 0.0, gam = 0.0, gam1 = a.gamma1, beta_k = 0.0, beta_k1 = 0.0, inv_b = 0.0, cpsi = 0.0;
-    const int ks = step_index(a);
-    if (mode == kModeStep) {
-        beta_k1 = a.tri_sub[ks];
-        // the chain already ended (breakdown recorded by an earlier launch)
-        if (!(beta_k1 >= a.cutoff) || a.flags[0] != 0) return;
-        const double alpha = a.tri_diag[ks - 1];
-        gam = ks >= 2 ? a.tri_diag[ks - 2] : a.gamma1;
-        delta = alpha - gam;
-        gam1 = alpha;
-        beta_k = ks >= 2 ? a.tri_sub[ks - 1] : 0.0;
-        inv_b = 1.0 / beta_k1;
-        if (a.psi_coef) cpsi = a.psi_coef[ks];
-    }
+    chain_next();
     {
         for (int i = tid; i < H.up.npal; i += NTHR) {
             pal_s[i] = H.up.pal[i];
@@ -154,6 +140,22 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
             for (int o2 = H.int_off[tid]; o2 < H.int_off[tid + 1]; ++o2) t += H.int_coef[o2];
             s_dsum[tid] = t;
         }
+    }
+    chain_wait();
+    const int mode = STEP ? (int)kModeStep : a.mode;
+    double delta = 0.0, gam = 0.0, gam1 = a.gamma1, beta_k = 0.0, beta_k1 = 0.0, inv_b = 0.0, cpsi = 0.0;
+    const int ks = step_index(a);
+    if (mode == kModeStep) {
+        beta_k1 = a.tri_sub[ks];
+        // the chain already ended (breakdown recorded by an earlier launch)
+        if (!(beta_k1 >= a.cutoff) || a.flags[0] != 0) return;
+        const double alpha = a.tri_diag[ks - 1];
+        gam = ks >= 2 ? a.tri_diag[ks - 2] : a.gamma1;
+        delta = alpha - gam;
+        gam1 = alpha;
+        beta_k = ks >= 2 ? a.tri_sub[ks - 1] : 0.0;
+        inv_b = 1.0 / beta_k1;
+        if (a.psi_coef) cpsi = a.psi_coef[ks];
     }
     if (tid == 0) {
         mbar_init(&s_bar[0], 1);
@@ -469,18 +471,15 @@ cudaError_t launch_tma_t(const HamDev &H, const RowArgs &a, int num_sms, cudaStr
                                  : row_tma_kernel<T, R, KMU, KMD, NTHR, MINB, CPT, PIPE, S32, false>;
     const int slot = tma_slot_elems(H.dup, sizeof(T));
     const size_t smem = (size_t)2 * R * slot * sizeof(T);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, NTHR, smem);
+    cudaError_t e = kernel_fit(reinterpret_cast<const void *>(k), NTHR, smem, &per_sm);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     const int64_t groups = (H.ddn + R - 1) / R;
     int64_t grid = (int64_t)num_sms * per_sm;
     if (grid > groups) grid = groups;
     if (grid < 1) grid = 1;
-    k<<<(int)grid, NTHR, smem, st>>>(H, a, slot);
-    return cudaGetLastError();
+    return launch_chained(k, (int)grid, NTHR, smem, st, H, a, slot);
 }
 
 cudaError_t launch_tma_f32(const HamDev &H, const RowArgs &a, int num_sms, const FastShape &s, cudaStream_t st);

@@ -127,11 +127,13 @@ __global__ void __launch_bounds__(NTMAX, MINB) sz_row_kernel(const SzDev S, cons
     uint32_t *db = reinterpret_cast<uint32_t *>(runs + S.nrun);
     int *seg = reinterpret_cast<int *>(db + S.ndiag);
     T *xs = reinterpret_cast<T *>(smem_raw + S.smem_lists);
+    chain_next();
     for (int t = threadIdx.x; t < nq; t += blockDim.x) qs[t] = S.quart[t];
     for (int t = threadIdx.x; t < S.nterm; t += blockDim.x) { h2[2 * t] = S.terms[t].h; h2[2 * t + 1] = -S.terms[t].h; }
     if (threadIdx.x == 0) h2[2 * S.nterm] = 0.0;
     for (int t = threadIdx.x; t < S.nrun; t += blockDim.x) runs[t] = S.runs[t];
 
+    chain_wait();
     const int ks = step_index(a);
     StepScalars sc;
     if (!step_scalars(a, ks, sc)) return;
@@ -326,11 +328,13 @@ __global__ void __launch_bounds__(NT, 1024 / NT) sz_wide_kernel(const SzDev S, c
     int *seg = reinterpret_cast<int *>(db + S.ndiag);
     T *xs = reinterpret_cast<T *>(smem_raw + S.smem_lists);         // own row, two buffers
     const int pitch = S.sec.pitch, tid = threadIdx.x;
+    chain_next();
     for (int t = tid; t < nq; t += NT) qs[t] = S.quart[t];
     for (int t = tid; t < S.nterm; t += NT) { h2[2 * t] = S.terms[t].h; h2[2 * t + 1] = -S.terms[t].h; }
     if (tid == 0) h2[2 * S.nterm] = 0.0;
     for (int t = tid; t < S.nrun; t += NT) runs[t] = S.runs[t];
 
+    chain_wait();
     const int ks = step_index(a);
     StepScalars sc;
     if (!step_scalars(a, ks, sc)) return;
@@ -500,9 +504,11 @@ __global__ void __launch_bounds__(kSzBlock) sz_row_simple_kernel(const SzDev S, 
     double *des = qs + nq;
     uint32_t *dbs = reinterpret_cast<uint32_t *>(des + S.ndiag);
     for (int t = threadIdx.x; t < S.nterm; t += blockDim.x) ts[t] = S.terms[t];
+    chain_next();
     for (int t = threadIdx.x; t < nq; t += blockDim.x) qs[t] = S.quart[t];
     for (int t = threadIdx.x; t < S.ndiag; t += blockDim.x) { des[t] = S.diag_e[t]; dbs[t] = S.diag_bit[t]; }
 
+    chain_wait();
     const int ks = step_index(a);
     StepScalars sc;
     if (!step_scalars(a, ks, sc)) return;
@@ -604,12 +610,10 @@ int sz_block(int maxlen, int most = kSzBlock)
 template <typename K>
 cudaError_t launch_one(K kern, int grid, int block, size_t smem, const SzDev &S, const RowArgs &a, cudaStream_t st)
 {
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
-    kern<<<grid, block, smem, st>>>(S, a);
-    return cudaGetLastError();
+    int per_sm = 0;      // allows the shared memory; the callers size the grid themselves
+    cudaError_t e = kernel_fit(reinterpret_cast<const void *>(kern), block, smem, &per_sm);
+    if (e != cudaSuccess) return e;
+    return launch_chained(kern, grid, block, smem, st, S, a);
 }
 
 }  // namespace
