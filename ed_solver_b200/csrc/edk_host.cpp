@@ -486,8 +486,8 @@ int fast_shape_for(edk_h *h, int dtype, const RowArgs &a, bool aligned, FastShap
         return EDK_OK;
     }
     char key[160];
-    std::snprintf(key, sizeof key, "%d:%lld:%lld:%d:%d:%d:%d", dtype, (long long)h->H.dup, (long long)h->H.ddn,
-                  h->H.up.ell_k, h->H.dn_kmax, h->H.nc, a.sum32);
+    std::snprintf(key, sizeof key, "%d:%lld:%lld:%d:%d:%d:%d:%d", dtype, (long long)h->H.dup, (long long)h->H.ddn,
+                  h->H.up.ell_k, h->H.dn_kmax, h->H.nc, a.sum32, h->H.hund);
     if (c->kernel_path == 0)
         for (const auto &kv : c->fast_by_shape)
             if (kv.first == key) {

@@ -119,6 +119,7 @@ struct RowArgs {
 // hops from L2-resident column tiles (edk_rows_tiled.cuh), with an FP32
 // scratch vector (RowArgs::scratch); variant 0 stages two row pairs per
 // up-pass block, 1 one pair.  Both need aligned column pairs.
+// Sectors with Hund terms (two impurity sites) take kinds 1 and 2.
 inline bool shape_needs_pairs(int kind) { return kind == 0 || kind == 2 || kind == 3 || kind == 5; }
 struct FastShape {
     int r = 0, kmu = 0, kmd = 0, variant = 0, kind = 0;

@@ -40,19 +40,37 @@ bool fast_rows_ok(const HamDev &H, int elem_bytes)
 {
     const int kmax = H.up.ell_k > H.dn_kmax ? H.up.ell_k : H.dn_kmax;
     const int64_t rowbytes = H.dup * (int64_t)elem_bytes;
-    return !H.hund && H.nc <= 2 && kmax <= 16 && rowbytes <= kMaxSmemBytes && H.up.packed &&
+    return H.nc <= 2 && kmax <= 16 && rowbytes <= kMaxSmemBytes && H.up.packed &&
            H.dup * H.ddn < (int64_t)1 << 31 && H.up.ell_k >= 0;
 }
 
 int fast_shapes(const HamDev &H, int elem_bytes, int num_sms, FastShape *out, int cap, int sum32)
 {
     if (!fast_rows_ok(H, elem_bytes)) return 0;
+    int n = 0;
+    if (H.hund) {
+        // Hund terms: kinds 1 and 2, as many blocks per SM as the staged rows allow
+        // (two buffers a block and up to 5.5 KB of tables).  FP64 H*v of two-orbital
+        // sectors, us, against the generic row kernel's: 2,944,656 states 66 (kind 2,
+        // 128 threads; 73 kind 1) / 137; 853,776 26 / 46; 213,444 9.6 / 17.2; FP32
+        // 2,944,656 47 / 124.  Below 2^17 states the shapes lie within the timing's
+        // noise (63,504: 5.1-5.5, generic 5.5), so one is taken untimed.
+        const int kmax = H.up.ell_k > H.dn_kmax ? H.up.ell_k : H.dn_kmax;
+        const int km = kmax <= 8 ? 8 : kmax <= 12 ? 12 : 16;
+        const int64_t need = 2 * (int64_t)tma_slot_elems(H.dup, elem_bytes) * elem_bytes + 5632;
+        static const int blocks1[5] = {3, 4, 7, 2, 1}, blocks2[3] = {2, 4, 1};
+        const bool small = H.dup * H.ddn < (int64_t)1 << 17;
+        for (int v = 0; v < 5 && n < cap && !(small && n > 0); ++v)
+            if (blocks1[v] * need <= 228 * 1024) out[n++] = FastShape{1, km, km, v, 1};
+        for (int v = 0; v < 3 && n < cap && !small && H.dup % 2 == 0; ++v)
+            if (blocks2[v] * need <= 228 * 1024) out[n++] = FastShape{1, km, km, v, 2};
+        return n;
+    }
     const int kmu = H.up.ell_k <= 8 ? 8 : 16;
     const int kmd = H.dn_kmax <= 4 ? 4 : H.dn_kmax <= 8 ? 8 : H.dn_kmax <= 12 ? 12 : 16;
     const int64_t rowbytes = H.dup * (int64_t)elem_bytes;
     int rs[3];
     const int nr = rows_allowed(elem_bytes, kmd, rs);
-    int n = 0;
     // the register-staged kernel reads column pairs: even rows only
     for (int variant = 0; variant < 3 && (H.dup % 2) == 0; ++variant) {
         // shared memory per block when 1, 2 or 4 blocks share an SM
@@ -125,6 +143,8 @@ int fast_shapes(const HamDev &H, int elem_bytes, int num_sms, FastShape *out, in
 cudaError_t launch_rows_fast(const HamDev &H, int dtype, const RowArgs &a, int num_sms, const FastShape &s,
                              cudaStream_t st)
 {
+    if (H.hund)
+        return dtype == EDK_F64 ? launch_hund_f64(H, a, num_sms, s, st) : launch_hund_f32(H, a, num_sms, s, st);
     if (s.kind == 3) return dtype == EDK_F32 ? launch_lean_f32(H, a, num_sms, s, st) : cudaErrorInvalidValue;
     if (s.kind == 5) return dtype == EDK_F32 ? launch_tiled_f32(H, a, num_sms, s, st) : cudaErrorInvalidValue;
     if (s.kind >= 1)

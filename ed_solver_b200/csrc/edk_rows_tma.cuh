@@ -99,7 +99,12 @@ __device__ __forceinline__ void row_middle(const T *src, int n, int &c16, int &c
 // slot: elements per staged-row slot (a multiple of 16 bytes, >= dup + 16/sizeof(T)).
 // STEP: the launch is a fused Lanczos step (mode kModeStep known at compile
 // time); otherwise the mode is read from the arguments.
-template <typename T, int R, int KMU, int KMD, int NTHR, int MINB, int CPT, bool PIPE, bool S32, bool STEP>
+// HUND: spin flip and pair hopping of two impurity sites (HAIMupdo.f90:1017-1129).
+// An element has at most one such term, where both spins' impurity sites hold
+// one electron each: x at the states with both electrons moved, reached through
+// the move tables; the row's part of it is prepared with the neighbour table.
+template <typename T, int R, int KMU, int KMD, int NTHR, int MINB, int CPT, bool PIPE, bool S32, bool STEP,
+          bool HUND = false>
 __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, const RowArgs a, const int slot)
 {
     static_assert(!S32 || sizeof(T) == 4, "FP32 hop sums are for FP32 vectors");
@@ -118,6 +123,8 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
     __shared__ double s_hd[2][R][KMD];
     __shared__ int s_row[2][R], s_cd[2][R], s_off[2][R];
     __shared__ double s_dd[2][R];
+    // HUND: neighbour rows, offset of the moved row (-1: no term), its sign
+    __shared__ int s_nd[2][R], s_hofs[2][R], s_hneg[2][R];
     __shared__ __align__(8) uint64_t s_bar[2];
     T *rowbuf = reinterpret_cast<T *>(smem_raw);   // [2][R][slot]
     const int dup = (int)H.dup;
@@ -192,6 +199,13 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
             s_dd[b][r] = H.dn.diag[rr];
             s_cd[b][r] = (int)H.dn.imp[rr];
             s_off[b][r] = (int)((reinterpret_cast<uintptr_t>(x + (int64_t)rr * dup) & 15) / sizeof(T));
+            if (HUND) {
+                const int cd = (int)H.dn.imp[rr];
+                const int32_t pd = cd == 1 || cd == 2 ? H.dn.move[2 * rr + cd - 1] : 0;
+                s_hofs[b][r] = pd ? ((pd > 0 ? pd : -pd) - 1) * dup : -1;
+                s_hneg[b][r] = pd < 0;
+                s_nd[b][r] = H.dn.ptr[rr + 1] - H.dn.ptr[rr];
+            }
         } else if (tid == kMeta + R) {
             // the bulk copies: one expect_tx for the group's total, then one copy per row
             uint32_t total = 0;
@@ -243,8 +257,9 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
         T vk[R][CPT], vm[R][CPT];
         int cu[CPT];
         double du[CPT];
+        int2 mv[CPT];              // HUND: the up electron's moves 0 -> 1 and 1 -> 0
     };
-    auto load = [&](int c, const int (&row)[R], const int (&nofs)[R][KMD], Ld &L) {
+    auto load = [&](int c, int b, const int (&row)[R], const int (&nofs)[R][KMD], Ld &L) {
 #pragma unroll
         for (int k = 0; k < KMU; ++k) {
             if (CPT == 2) {
@@ -258,7 +273,10 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
 #pragma unroll
         for (int r = 0; r < R; ++r)
 #pragma unroll
-            for (int f = 0; f < KMD; ++f) ld_cols(x + nofs[r][f] + c, keep, L.xd[r][f]);
+            for (int f = 0; f < KMD; ++f) {
+                if (HUND && f >= s_nd[b][r]) break;
+                ld_cols(x + (HUND ? s_nofs[b][r][f] : nofs[r][f]) + c, keep, L.xd[r][f]);
+            }
         if (mode == kModeStep) {
 #pragma unroll
             for (int r = 0; r < R; ++r) {
@@ -275,8 +293,15 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
             L.cu[e] = H.up.imp[c + e];
             L.du[e] = __ldg(upd + c + e);
         }
+        if (HUND) {
+#pragma unroll
+            for (int e = 0; e < CPT; ++e)
+                L.mv[e] = __ldg(reinterpret_cast<const int2 *>(H.up.move) + c + e);
+        }
     };
 
+    const double jj01 = HUND ? H.jj[1] : 0.0, jj10 = HUND ? H.jj[2] : 0.0;
+    const bool um01 = HUND && H.umask[1], um10 = HUND && H.umask[2];
     double s0 = 0.0, s1 = 0.0, s2 = 0.0;
     auto compute = [&](int c, int b, const int (&row)[R], const int (&cd)[R], const double (&dd)[R],
                        const T *(&xs)[R], const float (&hd32)[R][KMD], const Ld &L) {
@@ -287,6 +312,19 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
         for (int r = 0; r < R; ++r)
 #pragma unroll
             for (int e = 0; e < CPT; ++e) o[r][e] = xs[r][c + e];
+        // HUND: the up electron's move, and x where both moved (used last)
+        int hp[CPT];
+        T hx[R][CPT];
+        if (HUND) {
+#pragma unroll
+            for (int e = 0; e < CPT; ++e) {
+                hp[e] = L.cu[e] == 1 ? L.mv[e].x : L.cu[e] == 2 ? L.mv[e].y : 0;
+                const int ju = (hp[e] > 0 ? hp[e] : -hp[e]) - 1;
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    hx[r][e] = hp[e] && s_hofs[b][r] >= 0 ? __ldg(x + s_hofs[b][r] + ju) : T(0);
+            }
+        }
         // density terms, diagonal (FP64)
 #pragma unroll
         for (int r = 0; r < R; ++r)
@@ -335,6 +373,7 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
                     if (S32) {
                         d32[r][e] = fmaf(hd32[r][f], (float)L.xd[r][f][e], d32[r][e]);
                     } else {
+                        if (HUND && f >= s_nd[b][r]) continue;   // padding, as in the generic kernel
                         const double h = s_hd[b][r][f];
                         if (EXACT) acc[r][e] = hmadd<T>(acc[r][e], h, L.xd[r][f][e]);
                         else accd[r][e] = hmadd<T>(accd[r][e], h, L.xd[r][f][e]);
@@ -346,6 +385,19 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
 #pragma unroll
                 for (int e = 0; e < CPT; ++e)
                     acc[r][e] += S32 ? (double)u32[r][e] + (double)d32[r][e] : accd[r][e];
+        }
+        if (HUND) {
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int e = 0; e < CPT; ++e)
+                    if (s_hofs[b][r] >= 0 && hp[e]) {
+                        // pair hopping out of site 1, else the (0, 1) element
+                        const bool up1 = L.cu[e] == 2 && cd[r] == 2;
+                        if (!(up1 ? um10 : um01)) continue;
+                        const double t = fmul((double)hx[r][e], up1 ? jj10 : jj01);
+                        acc[r][e] = (hp[e] < 0) == (s_hneg[b][r] != 0) ? fadd(acc[r][e], t) : fsub(acc[r][e], t);
+                    }
         }
         // epilogue
 #pragma unroll
@@ -430,21 +482,21 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
             // the loads of the next columns in flight while these are computed
             Ld A, B;
             int c = tid * CPT;
-            if (c < dup) load(c, row, nofs, A);
+            if (c < dup) load(c, b, row, nofs, A);
             while (c < dup) {
                 const int c1 = c + STRIDE;
-                if (c1 < dup) load(c1, row, nofs, B);
+                if (c1 < dup) load(c1, b, row, nofs, B);
                 compute(c, b, row, cd, dd, xs, hd32, A);
                 if (c1 >= dup) break;
                 const int c2 = c1 + STRIDE;
-                if (c2 < dup) load(c2, row, nofs, A);
+                if (c2 < dup) load(c2, b, row, nofs, A);
                 compute(c1, b, row, cd, dd, xs, hd32, B);
                 c = c2;
             }
         } else {
             for (int c = tid * CPT; c < dup; c += STRIDE) {
                 Ld A;
-                load(c, row, nofs, A);
+                load(c, b, row, nofs, A);
                 compute(c, b, row, cd, dd, xs, hd32, A);
             }
         }
@@ -464,11 +516,11 @@ inline int tma_slot_elems(int64_t dup, int elem_bytes)
     return (int)((dup + v + v - 1) / v * v);
 }
 
-template <typename T, int R, int KMU, int KMD, int NTHR, int MINB, int CPT, bool PIPE, bool S32>
+template <typename T, int R, int KMU, int KMD, int NTHR, int MINB, int CPT, bool PIPE, bool S32, bool HUND = false>
 cudaError_t launch_tma_t(const HamDev &H, const RowArgs &a, int num_sms, cudaStream_t st)
 {
-    auto k = a.mode == kModeStep ? row_tma_kernel<T, R, KMU, KMD, NTHR, MINB, CPT, PIPE, S32, true>
-                                 : row_tma_kernel<T, R, KMU, KMD, NTHR, MINB, CPT, PIPE, S32, false>;
+    auto k = a.mode == kModeStep ? row_tma_kernel<T, R, KMU, KMD, NTHR, MINB, CPT, PIPE, S32, true, HUND>
+                                 : row_tma_kernel<T, R, KMU, KMD, NTHR, MINB, CPT, PIPE, S32, false, HUND>;
     const int slot = tma_slot_elems(H.dup, sizeof(T));
     const size_t smem = (size_t)2 * R * slot * sizeof(T);
     int per_sm = 0;
@@ -484,5 +536,7 @@ cudaError_t launch_tma_t(const HamDev &H, const RowArgs &a, int num_sms, cudaStr
 
 cudaError_t launch_tma_f32(const HamDev &H, const RowArgs &a, int num_sms, const FastShape &s, cudaStream_t st);
 cudaError_t launch_tma_f64(const HamDev &H, const RowArgs &a, int num_sms, const FastShape &s, cudaStream_t st);
-
+// the same with Hund terms (kinds 1 and 2, one row per group)
+cudaError_t launch_hund_f32(const HamDev &H, const RowArgs &a, int num_sms, const FastShape &s, cudaStream_t st);
+cudaError_t launch_hund_f64(const HamDev &H, const RowArgs &a, int num_sms, const FastShape &s, cudaStream_t st);
 }  // namespace edk

@@ -33,3 +33,21 @@
     EDK_TMA_MORE(float, 8, 12, S) EDK_TMA_MORE(float, 16, 12, S)                                             \
     EDK_TMA_KIND(float, 1, 9, 8, S, 2, 2, false) EDK_TMA_KIND(float, 1, 8, 9, S, 2, 2, false)                \
     EDK_TMA_KIND(float, 1, 9, 9, S, 2, 2, false)
+
+// kinds 1 and 2 with Hund terms: one row per group, columns not pipelined.
+// The move table and the moved row's element do not fit beside a second
+// column's loads in 128 registers (spills); more resident threads hide the
+// latency better.  853,776 states, two orbitals, FP64 H*v: 26.3-28.7 us at 64-80
+// registers against 36.5 us pipelined (256 threads, two blocks per SM).
+#define EDK_TMA_HUND(T, KM)                                                                                  \
+    if (s.kind == 1 && s.kmu == KM)                                                                          \
+        return s.variant == 0   ? launch_tma_t<T, 1, KM, KM, 256, 3, 1, false, false, true>(H, a, num_sms, st) \
+               : s.variant == 1 ? launch_tma_t<T, 1, KM, KM, 256, 4, 1, false, false, true>(H, a, num_sms, st) \
+               : s.variant == 2 ? launch_tma_t<T, 1, KM, KM, 128, 7, 1, false, false, true>(H, a, num_sms, st) \
+               : s.variant == 3 ? launch_tma_t<T, 1, KM, KM, 512, 2, 1, false, false, true>(H, a, num_sms, st) \
+                                : launch_tma_t<T, 1, KM, KM, 1024, 1, 1, false, false, true>(H, a, num_sms, st); \
+    if (s.kind == 2 && s.kmu == KM)                                                                          \
+        return s.variant == 0   ? launch_tma_t<T, 1, KM, KM, 256, 2, 2, false, false, true>(H, a, num_sms, st) \
+               : s.variant == 1 ? launch_tma_t<T, 1, KM, KM, 128, 4, 2, false, false, true>(H, a, num_sms, st) \
+                                : launch_tma_t<T, 1, KM, KM, 512, 1, 2, false, false, true>(H, a, num_sms, st);
+#define EDK_TMA_HUND_ALL(T) EDK_TMA_HUND(T, 8) EDK_TMA_HUND(T, 12) EDK_TMA_HUND(T, 16)
