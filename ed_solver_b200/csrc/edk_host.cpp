@@ -460,6 +460,15 @@ int sum32_for(const edk_h *h, int dtype)
     return dtype == EDK_F32 && c->fp32_sums && h->dim >= c->fp32_sums_min_dim && !h->sz ? 1 : 0;
 }
 
+// What a timed launch shape is kept under: all that the candidates depend on.
+std::string shape_key(const edk_h *h, int dtype, int sum32)
+{
+    char key[160];
+    std::snprintf(key, sizeof key, "%d:%lld:%lld:%d:%d:%d:%d:%d", dtype, (long long)h->H.dup, (long long)h->H.ddn,
+                  h->H.up.ell_k, h->H.dn_kmax, h->H.nc, sum32, h->H.hund);
+    return key;
+}
+
 // aligned: every vector of the call is aligned to twice the element size,
 // which the register-staged kernel (kind 0) needs; without it only the
 // bulk-copy kernel (kind 1) is a candidate, taken untimed and not remembered.
@@ -485,9 +494,7 @@ int fast_shape_for(edk_h *h, int dtype, const RowArgs &a, bool aligned, FastShap
         out = cand[0];
         return EDK_OK;
     }
-    char key[160];
-    std::snprintf(key, sizeof key, "%d:%lld:%lld:%d:%d:%d:%d:%d", dtype, (long long)h->H.dup, (long long)h->H.ddn,
-                  h->H.up.ell_k, h->H.dn_kmax, h->H.nc, a.sum32, h->H.hund);
+    const std::string key = shape_key(h, dtype, a.sum32);
     if (c->kernel_path == 0)
         for (const auto &kv : c->fast_by_shape)
             if (kv.first == key) {
@@ -1459,9 +1466,7 @@ int edk_h_launch_shape_chosen(const edk_h *h, int dtype, int fp32_sums, int32_t 
         out = h->fast_shape[slot];
         found = true;
     } else {
-        char key[160];
-        std::snprintf(key, sizeof key, "%d:%lld:%lld:%d:%d:%d:%d", dtype, (long long)h->H.dup, (long long)h->H.ddn,
-                      h->H.up.ell_k, h->H.dn_kmax, h->H.nc, s32);
+        const std::string key = shape_key(h, dtype, s32);
         for (const auto &kv : h->ctx->fast_by_shape)
             if (kv.first == key) { out = kv.second; found = true; }
     }
