@@ -59,7 +59,10 @@ __device__ __forceinline__ void block_sum(double (&v)[NQ], double (*red)[32])
 }
 
 // Writes this block's NQ partial sums; the last block to arrive sums all
-// partials in block order into `out` and returns true (in thread 0 only).
+// partials, in an order that only the grid and block sizes fix, into `out` and
+// (thread 0) `v`, and returns true (in thread 0 only).  The whole block reads
+// the partials: one warp, quantity after quantity, spent several microseconds
+// of L2 latency on the 300 to 1,000 blocks of a Lanczos step.
 template <int NQ>
 __device__ bool grid_sum(double (&v)[NQ], double *partials, unsigned *counter, double *out)
 {
@@ -76,20 +79,17 @@ __device__ bool grid_sum(double (&v)[NQ], double *partials, unsigned *counter, d
     __syncthreads();
     if (!last) return false;
     __threadfence();
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            double t = 0.0;
-            for (unsigned b = lane; b < gridDim.x; b += 32)
-                t += __ldcg(&partials[(size_t)b * NQ + q]);
+    for (int q = 0; q < NQ; ++q) v[q] = 0.0;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x)
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-            if (lane == 0) out[q] = t;
-        }
-    }
-    if (threadIdx.x == 0) *counter = 0u;
-    return threadIdx.x == 0;
+        for (int q = 0; q < NQ; ++q) v[q] += __ldcg(&partials[(size_t)b * NQ + q]);
+    block_sum<NQ>(v, red);
+    if (threadIdx.x != 0) return false;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) out[q] = v[q];
+    *counter = 0u;
+    return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -198,14 +198,10 @@ __device__ __forceinline__ uint2 ldu2(const uint32_t *p)
 // a difference of numbers of size beta^2 + delta^2 instead of |w|^2.
 // The step index of a launch: the argument, or the device counter.
 __device__ __forceinline__ int step_index(const RowArgs &a) { return a.kdev ? *a.kdev : a.k; }
-__device__ __forceinline__ double step_gamma(const RowArgs &a, int k)
+// sum: |s'|^2, <s',v'>, |v'|^2; g: the gamma above (StepScalars::gam1).
+__device__ __forceinline__ void lanczos_finalize(const RowArgs &a, int k, const double (&sum)[3], double g)
 {
-    return a.mode == kModeFirst ? a.gamma1 : a.tri_diag[k - 1];
-}
-__device__ __forceinline__ void lanczos_finalize(const RowArgs &a, int k)
-{
-    const double sss = a.sums_out[0], ssv = a.sums_out[1], svv = a.sums_out[2];
-    const double g = step_gamma(a, k);
+    const double sss = sum[0], ssv = sum[1], svv = sum[2];
     const double al = ssv + g * svv;
     const double de = al - g;
     const double b2 = sss - 2.0 * de * ssv + de * de * svv;
@@ -230,19 +226,22 @@ struct StepScalars {
     double delta = 0.0, gam = 0.0, gam1 = 0.0, beta_k = 0.0, beta_k1 = 0.0, inv_b = 0.0, cpsi = 0.0;
 };
 // false: a step launch after the chain ended (breakdown recorded earlier).
+// All loads are issued before the first test: one trip to L2, not four.
 __device__ __forceinline__ bool step_scalars(const RowArgs &a, int ks, StepScalars &sc)
 {
     sc.gam1 = a.gamma1;
     if (a.mode != kModeStep) return true;
-    sc.beta_k1 = a.tri_sub[ks];
-    if (!(sc.beta_k1 >= a.cutoff) || a.flags[0] != 0) return false;
-    const double alpha = a.tri_diag[ks - 1];
-    sc.gam = ks >= 2 ? a.tri_diag[ks - 2] : a.gamma1;
+    const double b1 = __ldcg(a.tri_sub + ks), b0 = __ldcg(a.tri_sub + ks - 1);
+    const double alpha = __ldcg(a.tri_diag + ks - 1), prev = __ldcg(a.tri_diag + (ks >= 2 ? ks - 2 : 0));
+    const int ended = __ldcg(a.flags);
+    if (a.psi_coef) sc.cpsi = a.psi_coef[ks];
+    if (!(b1 >= a.cutoff) || ended != 0) return false;
+    sc.gam = ks >= 2 ? prev : a.gamma1;
     sc.delta = alpha - sc.gam;
     sc.gam1 = alpha;
-    sc.beta_k = ks >= 2 ? a.tri_sub[ks - 1] : 0.0;
-    sc.inv_b = 1.0 / sc.beta_k1;
-    if (a.psi_coef) sc.cpsi = a.psi_coef[ks];
+    sc.beta_k1 = b1;
+    sc.beta_k = ks >= 2 ? b0 : 0.0;
+    sc.inv_b = 1.0 / b1;
     return true;
 }
 

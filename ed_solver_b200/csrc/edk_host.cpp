@@ -92,7 +92,13 @@ struct edk_ctx {
     size_t work_limit = 0;   // > 0: the largest Krylov workspace a pass may allocate (bytes)
     size_t tri_cap = 0;
     int reduce_grid = 0;
-    bool graphs = true;      // replay pairs of fused Lanczos steps as a CUDA graph
+    // Replay pairs of fused Lanczos steps as a CUDA graph.  Off: programmatic
+    // launches overlap one step's end with the next one's tables, which two-step
+    // graphs cut at every replay (us per step of a 160-step chain, graph / plain:
+    // 400 states 9.0 / 6.5, 63,504 10.1 / 9.2, 853,776 23.5 / 21.8, 11.8 million
+    // equal; graphs of 4 to 32 steps gain less than 0.7 us on pairs).  A graph's
+    // host time is the smaller one (about 1 us a step against 3.5 us).
+    bool graphs = false;
     cudaStream_t capture_stream = nullptr;   // private stream the graphs are captured on
     // pinned host copies of alpha, beta and the flags for the overlapped
     // convergence checks of Lanczos pass 1
@@ -747,8 +753,8 @@ int krylov_step(Krylov &K)
     return EDK_OK;
 }
 
-// Fused steps until K.k == target.  From step 2 on, when the context allows
-// graphs and no per-launch timing is recorded, pairs of steps run as one CUDA
+// Fused steps until K.k == target.  From step 2 on, when the context asks for
+// graphs, pairs of steps run as one CUDA
 // graph launch (captured once per Krylov run; the first steps, which also time
 // the row kernel's launch shapes, run as plain launches).
 int krylov_run(Krylov &K, int target)

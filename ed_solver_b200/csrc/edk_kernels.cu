@@ -123,20 +123,11 @@ __global__ void __launch_bounds__(512, 1) row_kernel(const HamDev H, const RowAr
     // step scalars: s = w_k - gamma_k v_k was stored by the previous launch;
     // delta_k = alpha_k - gamma_k; the new vector is s' = w_{k+1} - gamma_{k+1} v_{k+1}
     // with gamma_{k+1} = alpha_k
-    double delta = 0.0, gam = 0.0, gam1 = a.gamma1, beta_k = 0.0, beta_k1 = 0.0, inv_b = 0.0, cpsi = 0.0;
+    StepScalars sc;
     const int ks = step_index(a);
-    if (a.mode == kModeStep) {
-        beta_k1 = a.tri_sub[ks];
-        // the chain already ended (breakdown recorded by an earlier launch)
-        if (!(beta_k1 >= a.cutoff) || a.flags[0] != 0) return;
-        const double alpha = a.tri_diag[ks - 1];
-        gam = ks >= 2 ? a.tri_diag[ks - 2] : a.gamma1;
-        delta = alpha - gam;
-        gam1 = alpha;
-        beta_k = ks >= 2 ? a.tri_sub[ks - 1] : 0.0;
-        inv_b = 1.0 / beta_k1;
-        if (a.psi_coef) cpsi = a.psi_coef[ks];
-    }
+    if (!step_scalars(a, ks, sc)) return;
+    const double delta = sc.delta, gam = sc.gam, gam1 = sc.gam1, beta_k = sc.beta_k, beta_k1 = sc.beta_k1;
+    const double inv_b = sc.inv_b, cpsi = sc.cpsi;
 
     const uint32_t *__restrict__ ell = H.up.ell;
     const double *__restrict__ ellv = H.up.ell_val;
@@ -146,7 +137,7 @@ __global__ void __launch_bounds__(512, 1) row_kernel(const HamDev H, const RowAr
     const double *__restrict__ dnd = H.dn.diag;
     const double *__restrict__ icoef = H.int_coef;
 
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
     const int64_t ngroups = (ddn + R - 1) / R;
     for (int64_t g = blockIdx.x; g < ngroups; g += gridDim.x) {
         int row[R];
@@ -308,9 +299,9 @@ __global__ void __launch_bounds__(512, 1) row_kernel(const HamDev H, const RowAr
     }
     if (a.mode == kModeHv) return;
 
-    double v[4] = {s0, s1, s2, s3};
-    if (grid_sum<4>(v, a.partials, a.counter, a.sums_out))
-        if (a.mode == kModeFirst || a.mode == kModeStep) lanczos_finalize(a, ks);
+    double v[3] = {s0, s1, s2};
+    if (grid_sum<3>(v, a.partials, a.counter, a.sums_out))
+        if (a.mode == kModeFirst || a.mode == kModeStep) lanczos_finalize(a, ks, v, gam1);
 }
 
 // ---------------------------------------------------------------------------

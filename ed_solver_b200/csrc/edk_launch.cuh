@@ -7,7 +7,10 @@
 // coefficients -- before they wait for it), and what a launch asks the runtime
 // about a kernel is asked once per thread, kernel and block shape.  H*v of a
 // sector of 400 or 4,900 states called in a row: 6.1 us a call, 3.6 us now (the
-// host's part of a call).
+// host's part of a call).  A fused step of a 160-step chain, two-step graphs
+// before, programmatic launches with the first row group's tables ahead of the
+// wait now: 400 states 10.3 -> 6.6 us, 15,876 12.3 -> 8.0, 853,776 26.5 -> 21.8,
+// 2,944,656 55.7 -> 50.6.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstddef>

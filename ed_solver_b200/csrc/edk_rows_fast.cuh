@@ -80,34 +80,38 @@ __global__ void __launch_bounds__(NTHR, MINB) row_fast_kernel(const HamDev H, co
         const int ncoef = H.int_off[nio - 1];
         for (int i = threadIdx.x; i < ncoef; i += blockDim.x) s_icoef[i] = H.int_coef[i];
     }
+    const int64_t ngroups = (ddn + R - 1) / R;
+    // neighbour rows (offsets, values) of a group, padded with value 0 on the own
+    // row; the first group's before the wait (tables no kernel writes)
+    auto neighbours = [&](int64_t g) {
+        for (int t = threadIdx.x; t < R * KMD; t += blockDim.x) {
+            const int r = t / KMD, f = t % KMD;
+            const int64_t q = g * R + r;
+            const int rr = q < ddn ? H.row_order[q] : 0;
+            const int f0 = H.dn.ptr[rr], nd = H.dn.ptr[rr + 1] - f0;
+            const bool ok = f < nd;
+            s_nofs[r][f] = (ok ? H.dn.tgt[f0 + f] : rr) * dup;
+            s_hd[r][f] = ok ? H.dn.val[f0 + f] : 0.0;
+        }
+    };
+    if ((int64_t)blockIdx.x < ngroups) neighbours(blockIdx.x);
     chain_wait();
     // step scalars: s = w_k - gamma_k v_k was stored by the previous launch;
     // delta_k = alpha_k - gamma_k; the new vector is s' = w_{k+1} - gamma_{k+1} v_{k+1}
     // with gamma_{k+1} = alpha_k
-    double delta = 0.0, gam = 0.0, gam1 = a.gamma1, beta_k = 0.0, beta_k1 = 0.0, inv_b = 0.0, cpsi = 0.0;
+    StepScalars sc;
     const int ks = step_index(a);
-    if (a.mode == kModeStep) {
-        beta_k1 = a.tri_sub[ks];
-        // the chain already ended (breakdown recorded by an earlier launch)
-        if (!(beta_k1 >= a.cutoff) || a.flags[0] != 0) return;
-        const double alpha = a.tri_diag[ks - 1];
-        gam = ks >= 2 ? a.tri_diag[ks - 2] : a.gamma1;
-        delta = alpha - gam;
-        gam1 = alpha;
-        beta_k = ks >= 2 ? a.tri_sub[ks - 1] : 0.0;
-        inv_b = 1.0 / beta_k1;
-        if (a.psi_coef) cpsi = a.psi_coef[ks];
-    }
+    if (!step_scalars(a, ks, sc)) return;
+    const double delta = sc.delta, gam = sc.gam, gam1 = sc.gam1, beta_k = sc.beta_k, beta_k1 = sc.beta_k1;
+    const double inv_b = sc.inv_b, cpsi = sc.cpsi;
     const uint64_t keep = l2_keep(), stream = l2_stream();
     const uint32_t *__restrict__ ell = H.up.ell;
     const int K = H.up.ell_k;
-    const double *__restrict__ dnv = H.dn.val;
     const double *__restrict__ upd = H.up.diag;
     const double *__restrict__ dnd = H.dn.diag;
     const int ncfg = H.ncfg;
 
     double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-    const int64_t ngroups = (ddn + R - 1) / R;
     for (int64_t g = blockIdx.x; g < ngroups; g += gridDim.x) {
         int row[R], cd[R];
         double dd[R];
@@ -120,16 +124,7 @@ __global__ void __launch_bounds__(NTHR, MINB) row_fast_kernel(const HamDev H, co
             cd[r] = (int)H.dn.imp[rr];
         }
         __syncthreads();
-        // neighbour rows (offsets, values) of the group, padded with value 0 on the own row
-        for (int t = threadIdx.x; t < R * KMD; t += blockDim.x) {
-            const int r = t / KMD, f = t % KMD;
-            const int64_t q = g * R + r;
-            const int rr = q < ddn ? H.row_order[q] : 0;
-            const int f0 = H.dn.ptr[rr], nd = H.dn.ptr[rr + 1] - f0;
-            const bool ok = f < nd;
-            s_nofs[r][f] = (ok ? H.dn.tgt[f0 + f] : rr) * dup;
-            s_hd[r][f] = ok ? dnv[f0 + f] : 0.0;
-        }
+        if (g != blockIdx.x) neighbours(g);
         // stage the R rows interleaved: xs[c*R + r]
         {
             constexpr int V = 16 / sizeof(T);
@@ -293,9 +288,9 @@ __global__ void __launch_bounds__(NTHR, MINB) row_fast_kernel(const HamDev H, co
         }
     }
     if (a.mode == kModeHv) return;
-    double v[4] = {s0, s1, s2, 0.0};
-    if (grid_sum<4>(v, a.partials, a.counter, a.sums_out))
-        if (a.mode == kModeFirst || a.mode == kModeStep) lanczos_finalize(a, ks);
+    double v[3] = {s0, s1, s2};
+    if (grid_sum<3>(v, a.partials, a.counter, a.sums_out))
+        if (a.mode == kModeFirst || a.mode == kModeStep) lanczos_finalize(a, ks, v, gam1);
 }
 
 // Launch of one instance: grid = SMs x resident blocks, at most one block per

@@ -247,9 +247,9 @@ __global__ void __launch_bounds__(NT, MINB) row_lean_kernel(const HamDev H, cons
         }
     }
     if (mode == kModeHv) return;
-    double v[4] = {s0, s1, s2, 0.0};
-    if (grid_sum<4>(v, a.partials, a.counter, a.sums_out))
-        if (mode == kModeFirst || mode == kModeStep) lanczos_finalize(a, ks);
+    double v[3] = {s0, s1, s2};
+    if (grid_sum<3>(v, a.partials, a.counter, a.sums_out))
+        if (mode == kModeFirst || mode == kModeStep) lanczos_finalize(a, ks, v, sc.gam1);
 }
 
 // Dynamic shared memory of one block: the two interleaved rows.

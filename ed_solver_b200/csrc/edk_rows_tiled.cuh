@@ -376,9 +376,9 @@ __global__ void __launch_bounds__(256, 4) down_pass_kernel(const HamDev H, const
         }
     }
     if (mode == kModeHv) return;
-    double v[4] = {s0, s1, s2, 0.0};
-    if (grid_sum<4>(v, a.partials, a.counter, a.sums_out))
-        if (mode == kModeFirst || mode == kModeStep) lanczos_finalize(a, ks);
+    double v[3] = {s0, s1, s2};
+    if (grid_sum<3>(v, a.partials, a.counter, a.sums_out))
+        if (mode == kModeFirst || mode == kModeStep) lanczos_finalize(a, ks, v, sc.gam1);
 }
 
 // Pass 2 with four columns per thread: every vector access is one 16-byte
@@ -497,9 +497,9 @@ __global__ void __launch_bounds__(256, 3) down_pass4_kernel(const HamDev H, cons
         }
     }
     if (mode == kModeHv) return;
-    double v[4] = {s0, s1, s2, 0.0};
-    if (grid_sum<4>(v, a.partials, a.counter, a.sums_out))
-        if (mode == kModeFirst || mode == kModeStep) lanczos_finalize(a, ks);
+    double v[3] = {s0, s1, s2};
+    if (grid_sum<3>(v, a.partials, a.counter, a.sums_out))
+        if (mode == kModeFirst || mode == kModeStep) lanczos_finalize(a, ks, v, sc.gam1);
 }
 
 // variant & 7 -- 0: two row pairs per up-pass block when they fit, 1: one

@@ -97,8 +97,9 @@ __device__ __forceinline__ void row_middle(const T *src, int n, int &c16, int &c
 // T: element type; R: rows per group; KMU/KMD: up/down table-width bounds;
 // NTHR threads per block (one column each), at least MINB blocks per SM.
 // slot: elements per staged-row slot (a multiple of 16 bytes, >= dup + 16/sizeof(T)).
-// STEP: the launch is a fused Lanczos step (mode kModeStep known at compile
-// time); otherwise the mode is read from the arguments.
+// STEP: the launch is a fused Lanczos step (mode kModeStep); otherwise one of
+// the other modes, read from the arguments (an instance without the step's
+// loads: H*v of 41,409,225 states, odd rows, 650 -> 600 us).
 // HUND: spin flip and pair hopping of two impurity sites (HAIMupdo.f90:1017-1129).
 // An element has at most one such term, where both spins' impurity sites hold
 // one electron each: x at the states with both electrons moved, reached through
@@ -148,40 +149,16 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
             s_dsum[tid] = t;
         }
     }
-    chain_wait();
-    const int mode = STEP ? (int)kModeStep : a.mode;
-    double delta = 0.0, gam = 0.0, gam1 = a.gamma1, beta_k = 0.0, beta_k1 = 0.0, inv_b = 0.0, cpsi = 0.0;
-    const int ks = step_index(a);
-    if (mode == kModeStep) {
-        beta_k1 = a.tri_sub[ks];
-        // the chain already ended (breakdown recorded by an earlier launch)
-        if (!(beta_k1 >= a.cutoff) || a.flags[0] != 0) return;
-        const double alpha = a.tri_diag[ks - 1];
-        gam = ks >= 2 ? a.tri_diag[ks - 2] : a.gamma1;
-        delta = alpha - gam;
-        gam1 = alpha;
-        beta_k = ks >= 2 ? a.tri_sub[ks - 1] : 0.0;
-        inv_b = 1.0 / beta_k1;
-        if (a.psi_coef) cpsi = a.psi_coef[ks];
-    }
     if (tid == 0) {
         mbar_init(&s_bar[0], 1);
         mbar_init(&s_bar[1], 1);
         mbar_fence_init();
     }
-    __syncthreads();
-
-    const uint64_t keep = l2_keep(), stream = l2_stream();
-    const uint32_t *__restrict__ ell = H.up.ell;
-    const int K = H.up.ell_k;
-    const double *__restrict__ upd = H.up.diag;
-    const int ncfg = H.ncfg;
     const int64_t ngroups = (ddn + R - 1) / R;
 
     // Group g into buffer b: neighbour table and row metadata (threads below
-    // kMeta + R), the rows' aligned middles by bulk copy (thread kMeta + R)
-    // and their ragged ends by plain loads (threads from kRagged on).
-    auto prepare = [&](int64_t g, int b) {
+    // kMeta + R) ...
+    auto tables = [&](int64_t g, int b) {
         if (tid < kMeta) {
             const int r = tid / KMD, f = tid % KMD;
             const int64_t q = g * R + r;
@@ -206,7 +183,13 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
                 s_hneg[b][r] = pd < 0;
                 s_nd[b][r] = H.dn.ptr[rr + 1] - H.dn.ptr[rr];
             }
-        } else if (tid == kMeta + R) {
+        }
+    };
+    // ... the rows' aligned middles by bulk copy (thread kRagged - 1,
+    // of another warp than the tables of up to 31 entries) and their
+    // ragged ends by plain loads (threads from kRagged on).
+    auto copies = [&](int64_t g, int b) {
+        if (tid == kRagged - 1) {
             // the bulk copies: one expect_tx for the group's total, then one copy per row
             uint32_t total = 0;
             const T *src[R];
@@ -250,6 +233,28 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
         }
     };
 
+    // the first group's tables before the wait (no kernel writes them)
+    const bool any = (int64_t)blockIdx.x < ngroups;
+    if (any) tables(blockIdx.x, 0);
+    __syncthreads();
+    chain_wait();
+    if (any) copies(blockIdx.x, 0);
+    const int mode = STEP ? (int)kModeStep : a.mode;
+    StepScalars sc;
+    const int ks = step_index(a);
+    sc.gam1 = a.gamma1;
+    if (STEP && !step_scalars(a, ks, sc)) {
+        if (any && !mbar_wait(&s_bar[0], 0)) atomicExch(&a.flags[1], 2);   // no copy in flight at the exit
+        return;
+    }
+    const double delta = sc.delta, gam = sc.gam, gam1 = sc.gam1, beta_k = sc.beta_k, beta_k1 = sc.beta_k1;
+    const double inv_b = sc.inv_b, cpsi = sc.cpsi;
+    const uint64_t keep = l2_keep(), stream = l2_stream();
+    const uint32_t *__restrict__ ell = H.up.ell;
+    const int K = H.up.ell_k;
+    const double *__restrict__ upd = H.up.diag;
+    const int ncfg = H.ncfg;
+
     // per-column loads (the pipeline stage): CPT adjacent columns
     struct Ld {
         uint32_t ent[KMU][CPT];
@@ -277,7 +282,7 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
                 if (HUND && f >= s_nd[b][r]) break;
                 ld_cols(x + (HUND ? s_nofs[b][r][f] : nofs[r][f]) + c, keep, L.xd[r][f]);
             }
-        if (mode == kModeStep) {
+        if (STEP) {
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 const size_t i = (size_t)(row[r] >= 0 ? row[r] : 0) * dup + c;
@@ -420,7 +425,7 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
                     s0 += sd * sd; s1 += sd * v; s2 += v * v;
                 }
                 st_cs(y, st);
-            } else if (mode == kModeStep) {
+            } else if (STEP) {
                 T wt[CPT], vt[CPT];
 #pragma unroll
                 for (int e = 0; e < CPT; ++e) {
@@ -451,14 +456,16 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
         }
     };
 
-    if ((int64_t)blockIdx.x < ngroups) prepare(blockIdx.x, 0);
     __syncthreads();
     int it = 0;
     for (int64_t g = blockIdx.x; g < ngroups; g += gridDim.x, ++it) {
         const int b = it & 1;
         const int64_t gn = g + gridDim.x;
         // buffer b ^ 1 was last read in the previous group (before the barrier below)
-        if (gn < ngroups) prepare(gn, b ^ 1);
+        if (gn < ngroups) {
+            tables(gn, b ^ 1);
+            copies(gn, b ^ 1);
+        }
         int row[R], cd[R], nofs[R][KMD];
         double dd[R];
         float hd32[R][KMD];
@@ -503,9 +510,9 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
         __syncthreads();
     }
     if (mode == kModeHv) return;
-    double v[4] = {s0, s1, s2, 0.0};
-    if (grid_sum<4>(v, a.partials, a.counter, a.sums_out))
-        if (mode == kModeFirst || mode == kModeStep) lanczos_finalize(a, ks);
+    double v[3] = {s0, s1, s2};
+    if (grid_sum<3>(v, a.partials, a.counter, a.sums_out))
+        if (STEP || mode == kModeFirst) lanczos_finalize(a, ks, v, gam1);
 }
 
 // Staged-row slot of the kernel above: dup elements plus up to 15 bytes of

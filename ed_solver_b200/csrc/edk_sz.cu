@@ -132,7 +132,10 @@ __global__ void __launch_bounds__(NTMAX, MINB) sz_row_kernel(const SzDev S, cons
     for (int t = threadIdx.x; t < S.nterm; t += blockDim.x) { h2[2 * t] = S.terms[t].h; h2[2 * t + 1] = -S.terms[t].h; }
     if (threadIdx.x == 0) h2[2 * S.nterm] = 0.0;
     for (int t = threadIdx.x; t < S.nrun; t += blockDim.x) runs[t] = S.runs[t];
-
+    // the first row's lists before the wait (no kernel writes the tables they come from)
+    __syncthreads();
+    if (threadIdx.x < 32 && blockIdx.x < S.sec.nrows)
+        sz_row_lists<T>(S, S.sec.row_h[blockIdx.x], runs, rt, hv, seg, de, db, &n_diag);
     chain_wait();
     const int ks = step_index(a);
     StepScalars sc;
@@ -151,7 +154,7 @@ __global__ void __launch_bounds__(NTMAX, MINB) sz_row_kernel(const SzDev S, cons
         const int c0 = S.class_start[k], len = S.class_start[k + 1] - c0;
         const uint32_t base = S.sec.off_h[h];
         __syncthreads();                       // the previous row is done with the lists
-        if (threadIdx.x < 32) sz_row_lists<T>(S, h, runs, rt, hv, seg, de, db, &n_diag);
+        if (r != blockIdx.x && threadIdx.x < 32) sz_row_lists<T>(S, h, runs, rt, hv, seg, de, db, &n_diag);
         if (STAGE) stage_row<T>(xs, x + base, len);
         __syncthreads();
         const int nd = n_diag;
@@ -275,9 +278,9 @@ __global__ void __launch_bounds__(NTMAX, MINB) sz_row_kernel(const SzDev S, cons
         }
     }
     if (a.mode == kModeHv) return;
-    double v[4] = {s0, s1, s2, 0.0};
-    if (grid_sum<4>(v, a.partials, a.counter, a.sums_out))
-        if (a.mode == kModeFirst || a.mode == kModeStep) lanczos_finalize(a, ks);
+    double v[3] = {s0, s1, s2};
+    if (grid_sum<3>(v, a.partials, a.counter, a.sums_out))
+        if (a.mode == kModeFirst || a.mode == kModeStep) lanczos_finalize(a, ks, v, sc.gam1);
 }
 
 // One element global -> shared, asynchronous, where i < n (predicated, no branch).
@@ -333,7 +336,10 @@ __global__ void __launch_bounds__(NT, 1024 / NT) sz_wide_kernel(const SzDev S, c
     for (int t = tid; t < S.nterm; t += NT) { h2[2 * t] = S.terms[t].h; h2[2 * t + 1] = -S.terms[t].h; }
     if (tid == 0) h2[2 * S.nterm] = 0.0;
     for (int t = tid; t < S.nrun; t += NT) runs[t] = S.runs[t];
-
+    // the first row's lists before the wait (no kernel writes the tables they come from)
+    __syncthreads();
+    if (tid < 32 && blockIdx.x < S.sec.nrows)
+        sz_row_lists<T>(S, S.sec.row_h[blockIdx.x], runs, rt, hv, seg, de, db, &n_diag);
     chain_wait();
     const int ks = step_index(a);
     StepScalars sc;
@@ -358,7 +364,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) sz_wide_kernel(const SzDev S, c
 #pragma unroll
         for (int i = 0; i < kSlots; ++i) copy_async(xs + tid + i * NT, x + base + tid + i * NT, tid + i * NT, len);
         copy_commit();
-        if (tid < 32) sz_row_lists<T>(S, h, runs, rt, hv, seg, de, db, &n_diag);
+        if (r != blockIdx.x && tid < 32) sz_row_lists<T>(S, h, runs, rt, hv, seg, de, db, &n_diag);
         copy_wait<0>();
         __syncthreads();
         const int nd = n_diag;
@@ -488,9 +494,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) sz_wide_kernel(const SzDev S, c
         }
     }
     if (a.mode == kModeHv) return;
-    double v[4] = {s0, s1, s2, 0.0};
-    if (grid_sum<4>(v, a.partials, a.counter, a.sums_out))
-        if (a.mode == kModeFirst || a.mode == kModeStep) lanczos_finalize(a, ks);
+    double v[3] = {s0, s1, s2};
+    if (grid_sum<3>(v, a.partials, a.counter, a.sums_out))
+        if (a.mode == kModeFirst || a.mode == kModeStep) lanczos_finalize(a, ks, v, sc.gam1);
 }
 
 // Reference form: every state walks the whole term list (kernel path 1).
@@ -553,9 +559,9 @@ __global__ void __launch_bounds__(kSzBlock) sz_row_simple_kernel(const SzDev S, 
         }
     }
     if (a.mode == kModeHv) return;
-    double v[4] = {s0, s1, s2, 0.0};
-    if (grid_sum<4>(v, a.partials, a.counter, a.sums_out))
-        if (a.mode == kModeFirst || a.mode == kModeStep) lanczos_finalize(a, ks);
+    double v[3] = {s0, s1, s2};
+    if (grid_sum<3>(v, a.partials, a.counter, a.sums_out))
+        if (a.mode == kModeFirst || a.mode == kModeStep) lanczos_finalize(a, ks, v, sc.gam1);
 }
 
 // Gather form of the reference's scatter: every target state looks up its

@@ -356,7 +356,8 @@ class Context:
         self.check(lib().edk_ctx_set_kernel_path(self.h, int(path)), "edk_ctx_set_kernel_path")
 
     def set_graphs(self, enable: bool):
-        """Replay pairs of fused Lanczos steps as CUDA graphs (default on)."""
+        """Replay pairs of fused Lanczos steps as CUDA graphs (default off: plain
+        launches are faster on the device, graphs take less host time)."""
         self.check(lib().edk_ctx_set_graphs(self.h, int(bool(enable))), "set_graphs")
 
     def timing(self, enable: bool):
