@@ -5,26 +5,35 @@
 // compute_dynamic chain (green_class_compute_dynamic.f90:191-334) per item.
 // For the many small, uneven sectors of a finite-temperature solve those
 // chains are launch-bound when each Lanczos step is its own grid.  Here every
-// chain is a work item: a thread block takes the next item from an atomic
-// queue (items sorted largest first) and runs all of its Lanczos steps alone,
-// with block-level reductions only -- no block ever waits on another, so the
-// kernel has no spin loop.  Vectors written inside the kernel are re-read with
-// L2-coherent loads (ld.global.cg), never through the read-only path.
+// chain is a work item: a cluster of 1 to 16 thread blocks takes the next item
+// from an atomic queue (items sorted largest first) and runs all of its Lanczos
+// steps, each block the rows of its rank; one cluster barrier per step hands the
+// partial sums (in distributed shared memory) and the vectors on.  A cluster's
+// blocks are resident together and no cluster waits on another.  With one block
+// per chain a step of a 4,900-state sector took 200 us, the latency of 70 rows
+// one after the other, while a dozen chains left nine tenths of the SMs idle.
+// Vectors written inside the kernel are re-read with L2-coherent loads
+// (ld.global.cg), never through the read-only path.
+#include <cooperative_groups.h>
 #include "edk_device.cuh"
 
 namespace edk {
 
+namespace cg = cooperative_groups;
+
 template <typename T> __device__ __forceinline__ T ldcg(const T *p) { return __ldcg(p); }
 
-// (H x) for all rows of one sector by one block, in the reference's order of
-// terms per element, fused with the Lanczos epilogue of `mode`.
+// (H x) for the rows of one sector that fall to rank `rank` of `nrank` blocks,
+// in the reference's order of terms per element, fused with the Lanczos epilogue
+// of `mode`.  R consecutive rows are staged at a time and their elements shared
+// out over the threads; loads go four at a time ahead of the ordered sum.
 // npsi > 0 (step mode): psi[j] += cpsi[j] * v_{k+1} for j < npsi, the
 // accumulation of a recomputing pass 2.
-template <typename T, int R>
+template <typename T>
 __device__ void block_rows(const HamDev &H, int mode, const T *x, T *y, const T *vk, const T *vkm1, T *vout,
                            double delta, double gam, double gam1, double beta_k, double beta_k1, double inv_b,
-                           T *xs, const double *pal_s, double &s0, double &s1, double &s2, int npsi = 0,
-                           T *const *psi = nullptr, const double *cpsi = nullptr)
+                           T *xs, int R, int rank, int nrank, const double *pal_s, double &s0, double &s1, double &s2,
+                           int npsi = 0, T *const *psi = nullptr, const double *cpsi = nullptr)
 {
     const int64_t dup = H.dup, ddn = H.ddn;
     const uint32_t *ell = H.up.ell;
@@ -35,38 +44,58 @@ __device__ void block_rows(const HamDev &H, int mode, const T *x, T *y, const T 
     const double *dnd = H.dn.diag;
     const double *icoef = H.int_coef;
     const double *jj = H.jj;
-    const int nc = H.nc;
-    for (int64_t g0 = 0; g0 < ddn; g0 += R) {
-        int row[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) row[r] = g0 + r < ddn ? (int)(g0 + r) : -1;
+    const uint8_t *upi = H.up.imp, *dni = H.dn.imp;
+    const int32_t *ptr = H.dn.ptr, *tgt = H.dn.tgt, *ioff = H.int_off;
+    const int nc = H.nc, ncfg = H.ncfg;
+    const bool packed = H.up.packed, hund = H.hund;
+    constexpr int B = 4;
+    for (int64_t g0 = (int64_t)rank * R; g0 < ddn; g0 += (int64_t)nrank * R) {
+        const int nel = (int)((ddn - g0 < R ? ddn - g0 : R) * dup);
         __syncthreads();
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-            if (row[r] >= 0)
-                for (int64_t i = threadIdx.x; i < dup; i += blockDim.x) xs[r * dup + i] = ldcg(x + row[r] * dup + i);
+        for (int i = threadIdx.x; i < nel; i += blockDim.x) xs[i] = ldcg(x + g0 * dup + i);
         __syncthreads();
-        for (int64_t c = threadIdx.x; c < dup; c += blockDim.x) {
-            const int cu = H.up.imp[c];
-            const double du = upd[c];
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                if (row[r] < 0) continue;
-                const T xo = xs[r * dup + c];
-                const int cd = H.dn.imp[row[r]];
-                const int cfg = cu * H.ncfg + cd;
+        for (int el = threadIdx.x; el < nel; el += blockDim.x) {
+            const int r = el / (int)dup, c = el - r * (int)dup;
+            const int64_t row = g0 + r;
+            const T *xr = xs + (size_t)r * dup;
+            const int cu = __ldg(upi + c), cd = __ldg(dni + row);
+            const double du = __ldg(upd + c), dd = __ldg(dnd + row);
+            const int f0 = __ldg(ptr + row), f1 = __ldg(ptr + row + 1);
+            {
+                const T xo = xs[el];
+                const int cfg = cu * ncfg + cd;
                 double acc = 0.0;
-                for (int o = H.int_off[cfg]; o < H.int_off[cfg + 1]; ++o) acc = hmadd<T>(acc, icoef[o], xo);
-                acc = hmadd<T>(acc, fadd(du, dnd[row[r]]), xo);
-                for (int k = 0; k < K; ++k) {
-                    const uint32_t ent = ell[(int64_t)k * dup + c];
-                    const int64_t j = H.up.packed ? (int64_t)(ent & 0xFFFFFFu) : (int64_t)(int32_t)ent;
-                    const double h = H.up.packed ? pal_s[ent >> 24] : ellv[(int64_t)k * dup + c];
-                    acc = hmadd<T>(acc, h, xs[r * dup + j]);
+                for (int o = __ldg(ioff + cfg), o1 = __ldg(ioff + cfg + 1); o < o1; ++o)
+                    acc = hmadd<T>(acc, __ldg(icoef + o), xo);
+                acc = hmadd<T>(acc, fadd(du, dd), xo);
+                for (int k0 = 0; k0 < K; k0 += B) {
+                    T xv[B];
+                    double h[B];
+#pragma unroll
+                    for (int u = 0; u < B; ++u) {
+                        const int k = k0 + u < K ? k0 + u : K - 1;
+                        const uint32_t ent = __ldg(ell + (int64_t)k * dup + c);
+                        h[u] = packed ? pal_s[ent >> 24] : __ldg(ellv + (int64_t)k * dup + c);
+                        xv[u] = xr[packed ? (int64_t)(ent & 0xFFFFFFu) : (int64_t)(int32_t)ent];
+                    }
+#pragma unroll
+                    for (int u = 0; u < B; ++u)
+                        if (k0 + u < K) acc = hmadd<T>(acc, h[u], xv[u]);
                 }
-                for (int f = H.dn.ptr[row[r]]; f < H.dn.ptr[row[r] + 1]; ++f)
-                    acc = hmadd<T>(acc, dnv[f], ldcg(x + (int64_t)H.dn.tgt[f] * dup + c));
-                if (H.hund) {
+                for (int q0 = f0; q0 < f1; q0 += B) {
+                    T xv[B];
+                    double h[B];
+#pragma unroll
+                    for (int u = 0; u < B; ++u) {
+                        const int f = q0 + u < f1 ? q0 + u : f1 - 1;
+                        h[u] = __ldg(dnv + f);
+                        xv[u] = ldcg(x + (int64_t)__ldg(tgt + f) * dup + c);
+                    }
+#pragma unroll
+                    for (int u = 0; u < B; ++u)
+                        if (q0 + u < f1) acc = hmadd<T>(acc, h[u], xv[u]);
+                }
+                if (hund) {
                     // Hund spin flip and pair hopping (HAIMupdo.f90:1017-1129), gathers from x
                     for (int s1 = 0; s1 < nc; ++s1) {
                         const int b1u = (cu >> s1) & 1, b1d = (cd >> s1) & 1;
@@ -79,7 +108,7 @@ __device__ void block_rows(const HamDev &H, int mode, const T *x, T *y, const T 
                             if (b1u && b2d) { mu = s1 * (nc - 1) + (s2 < s1 ? s2 : s2 - 1); md = s2 * (nc - 1) + (s1 < s2 ? s1 : s1 - 1); }
                             else if (b1d && b2u) { mu = s2 * (nc - 1) + (s1 < s2 ? s1 : s1 - 1); md = s1 * (nc - 1) + (s2 < s1 ? s2 : s2 - 1); }
                             if (mu < 0) continue;
-                            const int32_t pu = H.up.move[c * H.nmove + mu], pd = H.dn.move[(int64_t)row[r] * H.nmove + md];
+                            const int32_t pu = H.up.move[c * H.nmove + mu], pd = H.dn.move[row * H.nmove + md];
                             if (pu == 0 || pd == 0) continue;
                             const int64_t ju = (pu > 0 ? pu : -pu) - 1, jdn = (pd > 0 ? pd : -pd) - 1;
                             const double t = fmul((double)ldcg(x + ju + jdn * dup), jj[s1 * nc + s2]);
@@ -92,7 +121,7 @@ __device__ void block_rows(const HamDev &H, int mode, const T *x, T *y, const T 
                             if (s2 == s1 || !H.umask[s1 * nc + s2]) continue;
                             if (((cu >> s2) & 1) || ((cd >> s2) & 1)) continue;
                             const int mi = s1 * (nc - 1) + (s2 < s1 ? s2 : s2 - 1);
-                            const int32_t pu = H.up.move[c * H.nmove + mi], pd = H.dn.move[(int64_t)row[r] * H.nmove + mi];
+                            const int32_t pu = H.up.move[c * H.nmove + mi], pd = H.dn.move[row * H.nmove + mi];
                             if (pu == 0 || pd == 0) continue;
                             const int64_t ju = (pu > 0 ? pu : -pu) - 1, jdn = (pd > 0 ? pd : -pd) - 1;
                             const double t = fmul((double)ldcg(x + ju + jdn * dup), jj[s1 * nc + s2]);
@@ -100,7 +129,7 @@ __device__ void block_rows(const HamDev &H, int mode, const T *x, T *y, const T 
                         }
                     }
                 }
-                const int64_t i = (int64_t)row[r] * dup + c;
+                const int64_t i = row * dup + c;
                 if (mode == kModeFirst) {
                     const double v = (double)xo;
                     const T st = (T)((double)acc - gam1 * v);
@@ -138,85 +167,123 @@ __device__ __forceinline__ void block_allreduce(double (&v)[NQ], double (*red)[3
     __syncthreads();
 }
 
-template <typename T, int R>
-__global__ void __launch_bounds__(512, 1) batch_kernel(const HamDev *hams, const BatchItem *items, int nitems,
-                                                    int *queue, T *work, int64_t maxdim, double cutoff)
+template <typename T, int MINB>
+__global__ void __launch_bounds__(512, MINB) batch_kernel(const HamDev *hams, const BatchItem *items, int nitems,
+                                                    int *queue, T *work, int64_t maxdim, int smem_elems, double cutoff)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *xs = reinterpret_cast<T *>(smem_raw);
     __shared__ double pal_s[256];
     __shared__ double red[3][32];
-    __shared__ double bc[4];
+    __shared__ double part[2][3];      // this block's sums, read by the whole cluster
+    __shared__ double bc[3];
     __shared__ int item_id;
-    T *vA = work + (size_t)blockIdx.x * 4 * maxdim;
+    __shared__ __align__(16) unsigned char s_ham[sizeof(HamDev)];
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = (int)cl.block_rank(), nrank = (int)cl.num_blocks(), tid = threadIdx.x;
+    const int first = rank * blockDim.x + tid, stride = nrank * blockDim.x;
+    T *vA = work + (size_t)(blockIdx.x / nrank) * 4 * maxdim;
     T *vB = vA + maxdim, *sA = vB + maxdim, *sB = sA + maxdim;
+    int turn = 0;
+    // Sums over the cluster, the same bits in every thread of it.  The barrier also
+    // orders the cluster's stores to the vectors before its loads that follow.  A
+    // block's sums of one call are overwritten two calls on, after the next barrier.
+    auto cluster_sum = [&](double (&v)[3]) {
+        block_sum<3>(v, red);
+        if (tid == 0)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) part[turn][q] = v[q];
+        cl.sync();
+        if (tid < 32) {
+            double t[3] = {0.0, 0.0, 0.0};
+            if (tid < nrank) {
+                const double *p = cl.map_shared_rank(&part[turn][0], tid);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) t[q] = p[q];
+            }
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) t[q] += __shfl_down_sync(0xffffffffu, t[q], o);
+                if (tid == 0) bc[q] = t[q];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 3; ++q) v[q] = bc[q];
+        turn ^= 1;
+    };
     for (;;) {
-        __syncthreads();
-        if (threadIdx.x == 0) item_id = atomicAdd(queue, 1);
-        __syncthreads();
-        const int it = item_id;
+        if (rank == 0 && tid == 0) item_id = atomicAdd(queue, 1);
+        cl.sync();
+        const int it = *cl.map_shared_rank(&item_id, 0);
+        cl.sync();                     // every block has read it; none reads another's memory after this
         if (it >= nitems) return;
         const BatchItem &b = items[it];
-        const HamDev &H = hams[b.ham];
+        for (int i = tid; i < (int)(sizeof(HamDev) / 4); i += blockDim.x)
+            reinterpret_cast<uint32_t *>(s_ham)[i] = reinterpret_cast<const uint32_t *>(hams + b.ham)[i];
+        __syncthreads();
+        const HamDev &H = *reinterpret_cast<const HamDev *>(s_ham);
         const T *start = static_cast<const T *>(b.start);
         if (H.up.packed)
-            for (int i = threadIdx.x; i < H.up.npal; i += blockDim.x) pal_s[i] = H.up.pal[i];
+            for (int i = tid; i < H.up.npal; i += blockDim.x) pal_s[i] = H.up.pal[i];
+        // rows staged at a time: this rank's share, as far as the shared memory goes
+        const int64_t share = (H.ddn + nrank - 1) / nrank, fit = smem_elems / H.dup;
+        const int R = (int)(fit < 1 ? 1 : fit < share ? fit : share);
         // |start|^2 and v1 = start / |start|
         double nv[3] = {0.0, 0.0, 0.0};
-        for (int64_t i = threadIdx.x; i < b.dim; i += blockDim.x) {
+        for (int64_t i = first; i < b.dim; i += stride) {
             const double t = (double)start[i];
             nv[0] += t * t;
         }
-        block_allreduce<3>(nv, red, bc);
+        cluster_sum(nv);
         const double nrm = sqrt(nv[0]);
         if (!(nv[0] >= b.cutoff_dynamic) || !(nrm >= cutoff)) {
-            if (threadIdx.x == 0) *b.done = 0;
+            if (first == 0) *b.done = 0;
             continue;
         }
         const double inv = 1.0 / nrm;
-        for (int64_t i = threadIdx.x; i < b.dim; i += blockDim.x) vB[i] = (T)((double)start[i] * inv);
-        if (threadIdx.x == 0) b.beta[0] = nrm;
-        __syncthreads();
+        for (int64_t i = first; i < b.dim; i += stride) vB[i] = (T)((double)start[i] * inv);
+        if (first == 0) b.beta[0] = nrm;
+        cl.sync();
         T *vk = vB, *vkm1 = vA, *s = sA, *sn = sB;
-        double alpha_prev = 0.0, gam_prev = b.gamma1, beta_prev = 0.0;
+        double alpha_prev = 0.0, gam_prev = b.gamma1, beta_prev = 0.0, beta_k1 = nrm;
         int n = 0;
         for (int k = 0; k < b.niter; ++k) {
             double acc[3] = {0.0, 0.0, 0.0};
             double gam1;
             if (k == 0) {
                 gam1 = b.gamma1;
-                block_rows<T, R>(H, kModeFirst, vk, s, nullptr, nullptr, nullptr, 0, 0, gam1, 0, 0, 0, xs, pal_s,
-                                 acc[0], acc[1], acc[2]);
+                block_rows<T>(H, kModeFirst, vk, s, nullptr, nullptr, nullptr, 0, 0, gam1, 0, 0, 0, xs, R, rank, nrank,
+                              pal_s, acc[0], acc[1], acc[2]);
             } else {
-                const double beta_k1 = b.beta[k];
                 if (!(beta_k1 >= cutoff)) break;
                 const double delta = alpha_prev - gam_prev;
                 gam1 = alpha_prev;
-                block_rows<T, R>(H, kModeStep, s, sn, vk, k >= 2 ? vkm1 : nullptr, vkm1, delta, gam_prev, gam1,
-                                 beta_prev, beta_k1, 1.0 / beta_k1, xs, pal_s, acc[0], acc[1], acc[2]);
+                block_rows<T>(H, kModeStep, s, sn, vk, k >= 2 ? vkm1 : nullptr, vkm1, delta, gam_prev, gam1, beta_prev,
+                              beta_k1, 1.0 / beta_k1, xs, R, rank, nrank, pal_s, acc[0], acc[1], acc[2]);
                 T *t1 = vk; vk = vkm1; vkm1 = t1;        // v_{k+1} was written over v_{k-1}
                 T *t2 = s; s = sn; sn = t2;
             }
-            __threadfence_block();
-            block_allreduce<3>(acc, red, bc);
+            cluster_sum(acc);
             // coefficients of this iteration (same formulas as lanczos_finalize)
             const double g = gam1;
             const double al = acc[1] + g * acc[2];
             const double de = al - g;
             const double b2 = acc[0] - 2.0 * de * acc[1] + de * de * acc[2];
             const double ww = acc[0] + 2.0 * g * acc[1] + g * g * acc[2];
-            double be = (b2 > 0.0 && b2 > 1e-28 * ww && isfinite(b2)) ? sqrt(b2) : 0.0;
-            if (threadIdx.x == 0) {
+            const double be = (b2 > 0.0 && b2 > 1e-28 * ww && isfinite(b2)) ? sqrt(b2) : 0.0;
+            if (first == 0) {
                 b.alpha[k] = isfinite(al) ? al : 0.0;
                 b.beta[k + 1] = be;
             }
-            if (k >= 1) beta_prev = b.beta[k];
+            if (k >= 1) beta_prev = beta_k1;
+            beta_k1 = be;
             gam_prev = (k == 0) ? b.gamma1 : alpha_prev;
             alpha_prev = al;
             n = k + 1;
-            __syncthreads();
         }
-        if (threadIdx.x == 0) *b.done = n;
+        if (first == 0) *b.done = n;
     }
 }
 
@@ -357,15 +424,15 @@ __global__ void __launch_bounds__(512, 1) gs_batch_kernel(const HamDev *hams, co
             double gam1;
             if (k == 0) {
                 gam1 = 0.0;
-                block_rows<T, R>(H, kModeFirst, V[0], S[0], nullptr, nullptr, nullptr, 0, 0, gam1, 0, 0, 0, xs,
+                block_rows<T>(H, kModeFirst, V[0], S[0], nullptr, nullptr, nullptr, 0, 0, gam1, 0, 0, 0, xs, R, 0, 1,
                                  pal_s, acc[0], acc[1], acc[2]);
             } else {
                 const double beta_k1 = b.beta[k];
                 const double delta = alpha_prev - gam_prev;
                 gam1 = alpha_prev;
                 for (int j = 0; j < npsi; ++j) cps[j] = b.coef[(size_t)j * b.niter_max + k];
-                block_rows<T, R>(H, kModeStep, S[(k - 1) & 1], S[k & 1], V[(k - 1) & 1], k >= 2 ? V[k & 1] : nullptr,
-                                 V[k & 1], delta, gam_prev, gam1, beta_prev, beta_k1, 1.0 / beta_k1, xs, pal_s, acc[0],
+                block_rows<T>(H, kModeStep, S[(k - 1) & 1], S[k & 1], V[(k - 1) & 1], k >= 2 ? V[k & 1] : nullptr,
+                                 V[k & 1], delta, gam_prev, gam1, beta_prev, beta_k1, 1.0 / beta_k1, xs, R, 0, 1, pal_s, acc[0],
                                  acc[1], acc[2], npsi, psi, cps);
             }
             __threadfence_block();
@@ -458,46 +525,81 @@ cudaError_t launch_gs_batch(int R, const HamDev *hams, const GsItem *items, int 
 
 // ---------------------------------------------------------------------------
 
-template <typename T, int R>
-static cudaError_t launch_batch_t(const HamDev *hams, const BatchItem *items, int nitems, int *queue, void *work,
-                                  int64_t maxdim, int64_t maxdup, double cutoff, int grid, int block, cudaStream_t st)
+// Shared memory of a block: 32 KB of staged rows (four 512-thread blocks share an
+// SM), or the longest row.
+static size_t batch_smem(int elem_bytes, int64_t maxdup)
 {
-    auto k = batch_kernel<T, R>;
-    const size_t smem = (size_t)R * maxdup * sizeof(T);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem ? smem : 16));
-    if (e != cudaSuccess) return e;
-    k<<<grid, block, smem, st>>>(hams, items, nitems, queue, static_cast<T *>(work), maxdim, cutoff);
-    return cudaGetLastError();
+    const size_t row = (size_t)maxdup * elem_bytes;
+    return row > 32768 ? row : 32768;
 }
 
-cudaError_t launch_batch(int dtype, int R, const HamDev *hams, const BatchItem *items, int nitems, int *queue,
+// Wide clusters serve few chains, one block per SM: 128 registers (12 chains of
+// 4,900 states, 100 steps: 1.25 ms, 1.43 ms with 64).  One or two blocks per chain
+// serve many, two 512-thread blocks per SM: 64 registers (300 chains: 6.0 ms, 6.6 ms
+// with 128; 180 chains of 213,444 states 122 and 147 ms).  With one block per chain
+// and a row at a time these took 20, 26 and 262 ms.
+template <typename T> using BatchFn = void (*)(const HamDev *, const BatchItem *, int, int *, T *, int64_t, int, double);
+template <typename T> static BatchFn<T> batch_fn(int cluster)
+{
+    return cluster <= 2 ? batch_kernel<T, 2> : batch_kernel<T, 1>;
+}
+
+template <typename T>
+static cudaError_t batch_config(int cluster, int64_t maxdup, int grid, int block, cudaStream_t st,
+                                cudaLaunchAttribute *at, cudaLaunchConfig_t *cfg)
+{
+    auto k = batch_fn<T>(cluster);
+    const size_t smem = batch_smem(sizeof(T), maxdup);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+    if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = (unsigned)cluster;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    *cfg = cudaLaunchConfig_t{};
+    cfg->gridDim = dim3((unsigned)grid);
+    cfg->blockDim = dim3((unsigned)block);
+    cfg->dynamicSmemBytes = smem;
+    cfg->stream = st;
+    cfg->attrs = at;
+    cfg->numAttrs = 1;
+    return e;
+}
+
+template <typename T>
+static cudaError_t launch_batch_t(int cluster, const HamDev *hams, const BatchItem *items, int nitems, int *queue,
+                                  void *work, int64_t maxdim, int64_t maxdup, double cutoff, int grid, int block,
+                                  cudaStream_t st)
+{
+    cudaLaunchAttribute at;
+    cudaLaunchConfig_t cfg;
+    cudaError_t e = batch_config<T>(cluster, maxdup, grid, block, st, &at, &cfg);
+    if (e != cudaSuccess) return e;
+    return cudaLaunchKernelEx(&cfg, batch_fn<T>(cluster), hams, items, nitems, queue, static_cast<T *>(work), maxdim,
+                              (int)(cfg.dynamicSmemBytes / sizeof(T)), cutoff);
+}
+
+cudaError_t launch_batch(int dtype, int cluster, const HamDev *hams, const BatchItem *items, int nitems, int *queue,
                          void *work, int64_t maxdim, int64_t maxdup, double cutoff, int grid, int block,
                          cudaStream_t st)
 {
-    if (dtype == EDK_F64) {
-        if (R == 4) return launch_batch_t<double, 4>(hams, items, nitems, queue, work, maxdim, maxdup, cutoff, grid, block, st);
-        if (R == 2) return launch_batch_t<double, 2>(hams, items, nitems, queue, work, maxdim, maxdup, cutoff, grid, block, st);
-        return launch_batch_t<double, 1>(hams, items, nitems, queue, work, maxdim, maxdup, cutoff, grid, block, st);
-    }
-    if (R == 4) return launch_batch_t<float, 4>(hams, items, nitems, queue, work, maxdim, maxdup, cutoff, grid, block, st);
-    if (R == 2) return launch_batch_t<float, 2>(hams, items, nitems, queue, work, maxdim, maxdup, cutoff, grid, block, st);
-    return launch_batch_t<float, 1>(hams, items, nitems, queue, work, maxdim, maxdup, cutoff, grid, block, st);
+    return dtype == EDK_F64
+               ? launch_batch_t<double>(cluster, hams, items, nitems, queue, work, maxdim, maxdup, cutoff, grid, block, st)
+               : launch_batch_t<float>(cluster, hams, items, nitems, queue, work, maxdim, maxdup, cutoff, grid, block, st);
 }
 
-int batch_max_blocks_per_sm(int dtype, int R, int block, int64_t maxdup)
+int batch_max_clusters(int dtype, int cluster, int block, int64_t maxdup)
 {
+    cudaLaunchAttribute at;
+    cudaLaunchConfig_t cfg;
     int n = 0;
-    const size_t smem = (size_t)R * maxdup * (dtype == EDK_F64 ? 8 : 4);
-    cudaError_t e;
-    if (dtype == EDK_F64)
-        e = R == 4 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_kernel<double, 4>, block, smem)
-          : R == 2 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_kernel<double, 2>, block, smem)
-                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_kernel<double, 1>, block, smem);
-    else
-        e = R == 4 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_kernel<float, 4>, block, smem)
-          : R == 2 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_kernel<float, 2>, block, smem)
-                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_kernel<float, 1>, block, smem);
-    return e == cudaSuccess ? n : 0;
+    cudaError_t e = dtype == EDK_F64 ? batch_config<double>(cluster, maxdup, cluster, block, nullptr, &at, &cfg)
+                                     : batch_config<float>(cluster, maxdup, cluster, block, nullptr, &at, &cfg);
+    if (e == cudaSuccess)
+        e = dtype == EDK_F64 ? cudaOccupancyMaxActiveClusters(&n, batch_fn<double>(cluster), &cfg)
+                             : cudaOccupancyMaxActiveClusters(&n, batch_fn<float>(cluster), &cfg);
+    if (e == cudaSuccess) return n;
+    (void)cudaGetLastError();
+    return 0;
 }
 
 }  // namespace edk

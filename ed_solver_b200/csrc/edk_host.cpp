@@ -129,7 +129,7 @@ struct edk_ctx {
     // buffers of the other drivers (edk_internal_scratch), at most 256 MB each
     // between calls; edk_ctx_trim gives them back
     DevBuf scratch[3];
-    struct BatchShape { int block, R, per_sm; };
+    struct BatchShape { int block, cluster, clusters; };   // clusters: resident at a time
     std::vector<std::pair<std::string, BatchShape>> batch_tuned;
     // fast-kernel launch shape timed per sector shape (element type, dim_up,
     // dim_dn, table widths, impurity sites): a rebuilt Hamiltonian of the same
@@ -2196,20 +2196,23 @@ extern "C" int edk_green_batch(edk_ctx *c, int dtype, int32_t nchain, const edk_
     const size_t es = dtype == EDK_F64 ? 8 : 4;
 
     // ---- autotune the launch shape for this problem class ----
+    // (the number of chains, to a power of two: it decides how many blocks one gets)
+    int nclass = 0;
+    while ((1 << nclass) < nchain && nclass < 10) ++nclass;
     char key[96];
-    snprintf(key, sizeof key, "%d:%lld:%lld", dtype, (long long)maxdup, (long long)maxdim);
+    snprintf(key, sizeof key, "%d:%lld:%lld:%d", dtype, (long long)maxdup, (long long)maxdim, nclass);
     edk_ctx::BatchShape shape{0, 0, 0};
     for (auto &kv : c->batch_tuned)
         if (kv.first == key) shape = kv.second;
     auto run = [&](const edk_ctx::BatchShape &s, int nitems, double *ms) -> int {
-        const int grid = c->num_sms * s.per_sm;
-        int r2 = c->cuda(c->b_work.ensure(es * 4 * (size_t)maxdim * grid), "alloc batch workspace");
+        const int nclus = std::min(s.clusters, nitems), grid = nclus * s.cluster;
+        int r2 = c->cuda(c->b_work.ensure(es * 4 * (size_t)maxdim * nclus), "alloc batch workspace");
         if (r2) return r2;
         r2 = c->cuda(cudaMemsetAsync(c->b_queue.p, 0, sizeof(int), st), "memset");
         if (r2) return r2;
         cudaEvent_t a = c->get_event(), b = c->get_event();
         cudaEventRecord(a, st);
-        r2 = c->cuda(launch_batch(dtype, s.R, c->b_hams.as<HamDev>(), c->b_items.as<BatchItem>(), nitems,
+        r2 = c->cuda(launch_batch(dtype, s.cluster, c->b_hams.as<HamDev>(), c->b_items.as<BatchItem>(), nitems,
                                   c->b_queue.as<int>(), c->b_work.p, maxdim, maxdup, 1e-25, grid, s.block, st),
                      "batch kernel");
         c->launches++;
@@ -2224,25 +2227,22 @@ extern "C" int edk_green_batch(edk_ctx *c, int dtype, int32_t nchain, const edk_
     };
     int tuned = 0;
     if (shape.block == 0) {
-        // candidates: block size x rows per group x blocks per SM, timed on the
-        // largest items with the chain length cut to 6 steps
+        // candidates: block size x blocks per chain, timed on the largest items with
+        // the chain length cut to 6 steps
         const int nsample = std::min<int>(nchain, c->num_sms * 2);
         std::vector<BatchItem> sample(items.begin(), items.begin() + nsample);
         for (auto &b : sample) b.niter = std::min<int32_t>(b.niter, 6);
         if ((rc = c->cuda(upload(c->b_items, sample, st), "upload sample"))) return rc;
         double best = 1e300;
-        for (int block : {128, 256, 512})
-            for (int R : {1, 2, 4}) {
-                if ((int64_t)R * maxdup * (int64_t)es > 96 * 1024) continue;
-                const int occ = batch_max_blocks_per_sm(dtype, R, block, maxdup);
-                for (int per_sm : {1, 2, 4}) {
-                    if (per_sm > occ) continue;
-                    edk_ctx::BatchShape s{block, R, per_sm};
-                    double ms = 0;
-                    if ((rc = run(s, nsample, &ms))) return rc;
-                    ++tuned;
-                    if (ms < best) { best = ms; shape = s; }
-                }
+        for (int cluster : {1, 2, 4, 8, 16})
+            for (int block : {128, 256, 512}) {
+                const int active = batch_max_clusters(dtype, cluster, block, maxdup);
+                if (active < 1) continue;
+                edk_ctx::BatchShape s{block, cluster, active};
+                double ms = 0;
+                if ((rc = run(s, nsample, &ms))) return rc;
+                ++tuned;
+                if (ms < best) { best = ms; shape = s; }
             }
         if (shape.block == 0) return c->fail(EDK_ERR_UNSUPPORTED, "no batch launch shape fits");
         c->batch_tuned.push_back({key, shape});
@@ -2286,8 +2286,8 @@ extern "C" int edk_green_batch(edk_ctx *c, int dtype, int32_t nchain, const edk_
         stats->chains = nchain;
         stats->kernel_ms = ms;
         stats->block = shape.block;
-        stats->rows = shape.R;
-        stats->blocks_per_sm = shape.per_sm;
+        stats->rows = 1;                              // rows a thread sums at a time
+        stats->blocks_per_sm = std::max(1, std::min(shape.clusters, nchain) * shape.cluster / c->num_sms);
         stats->tuned_shapes = tuned;
     }
     return EDK_OK;

@@ -147,10 +147,11 @@ struct BatchItem {
     double *beta;            // niter + 1: beta[0] = |start|, beta[k] couples k-1,k
     int32_t *done;           // steps completed (0 if |start|^2 < cutoff_dynamic)
 };
-cudaError_t launch_batch(int dtype, int R, const HamDev *hams, const BatchItem *items, int nitems, int *queue,
+cudaError_t launch_batch(int dtype, int cluster, const HamDev *hams, const BatchItem *items, int nitems, int *queue,
                          void *work, int64_t maxdim, int64_t maxdup, double cutoff, int grid, int block,
                          cudaStream_t st);
-int batch_max_blocks_per_sm(int dtype, int R, int block, int64_t maxdup);
+// clusters of the batched kernel that are resident at a time (0: none)
+int batch_max_clusters(int dtype, int cluster, int block, int64_t maxdup);
 
 // The ground state of one small FP64 sector in a batched launch (edk_batch.cu).
 // Pass 1: up to niter_max Lanczos steps from the table start vector with the
