@@ -98,8 +98,11 @@ int fast_shapes(const HamDev &H, int elem_bytes, int num_sms, FastShape *out, in
         for (int i = 0; i < nr2 && n < cap; ++i)
             if (feasible(rs[i], variant)) out[n++] = FastShape{rs[i], kmu, kmd, variant, 1};
     // kind 2 (instantiated for down-table bounds 8 and 12, and in FP32 with
-    // one row per group for tables exactly 9 wide): variants 0, 1, 3 (768
-    // threads, one block per SM) and 4 (640 threads, one block per SM)
+    // one row per group for tables exactly 9 wide): variants 0, 1, 2, 3 (768
+    // threads, one block per SM) and 4 (640 threads, one block per SM).  Variant 2
+    // (four 128-thread blocks, rows up to 3,500 FP64 elements) evens out the last
+    // wave: 2,944,656 states, FP64 H*v 36.2 us (40.1 the best other shape), step
+    // 53.5 (55.5); 11.8 million, where three blocks fit, 168 against 151 for variant 1
     if ((kmd == 8 || kmd == 12) && (H.dup % 2) == 0) {
         const int kmu9 = elem_bytes == 4 && H.up.ell_k == 9 ? 9 : kmu;
         const int kmd9 = elem_bytes == 4 && H.dn_kmax == 9 ? 9 : kmd;
@@ -110,8 +113,8 @@ int fast_shapes(const HamDev &H, int elem_bytes, int num_sms, FastShape *out, in
             int ku = r == 1 ? kmu9 : kmu, kd = r == 1 ? kmd9 : kmd;
             // exact-9 instances: (9, 8), (8, 9), (9, 9)
             if ((ku == 9 && kd == 12) || (kd == 9 && ku == 16)) { ku = kmu; kd = kmd; }
-            for (int variant : {0, 1, 3, 4})
-                if (n < cap && feasible(r, variant >= 3 ? 0 : variant)) out[n++] = FastShape{r, ku, kd, variant, 2};
+            for (int variant : {0, 1, 2, 3, 4})
+                if (n < cap && !(variant == 2 && (sum32 || r > 1)) && feasible(r, variant >= 3 ? 0 : variant)) out[n++] = FastShape{r, ku, kd, variant, 2};
         }
     }
     // kind 3, the lean FP32 kernel (FP32 hop sums only): two interleaved rows

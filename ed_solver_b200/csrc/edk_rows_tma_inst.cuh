@@ -14,6 +14,7 @@
     if (s.kind == KIND && s.r == R && s.kmu == KMU && s.kmd == KMD)                                          \
         return s.variant == 0   ? launch_tma_t<T, R, KMU, KMD, 512, 1, CPT, PIPE, S>(H, a, num_sms, st)      \
                : s.variant == 1 ? launch_tma_t<T, R, KMU, KMD, 256, 2, CPT, PIPE, S>(H, a, num_sms, st)      \
+               : s.variant == 2 ? launch_tma_t<T, R, KMU, KMD, 128, 4, CPT, PIPE, S>(H, a, num_sms, st)      \
                : s.variant == 3 ? launch_tma_t<T, R, KMU, KMD, 768, 1, CPT, PIPE, S>(H, a, num_sms, st)      \
                                 : launch_tma_t<T, R, KMU, KMD, 640, 1, CPT, PIPE, S>(H, a, num_sms, st);
 // kind 2 (two columns per thread): rows per group 2 or 1
