@@ -2144,7 +2144,7 @@ extern "C" int edk_green_batch(edk_ctx *c, int dtype, int32_t nchain, const edk_
         if (stats) { stats->steps = steps; stats->chains = nchain; }
         return EDK_OK;
     }
-    // ---- persistent work queue ----
+    // ---- persistent work queue (a cluster of blocks per chain) ----
     std::vector<const edk_h *> hs;
     std::vector<HamDev> hd;
     std::vector<BatchItem> items(nchain);
@@ -2236,7 +2236,8 @@ extern "C" int edk_green_batch(edk_ctx *c, int dtype, int32_t nchain, const edk_
         double best = 1e300;
         for (int cluster : {1, 2, 4, 8, 16})
             for (int block : {128, 256, 512}) {
-                const int active = batch_max_clusters(dtype, cluster, block, maxdup);
+                // each resident chain holds four work vectors
+                const int active = std::min(batch_max_clusters(dtype, cluster, block, maxdup), 4 * c->num_sms);
                 if (active < 1) continue;
                 edk_ctx::BatchShape s{block, cluster, active};
                 double ms = 0;

@@ -326,9 +326,9 @@ int edk_block_lanczos(edk_h *h, const edk_block_opts *opts, double *E_host, void
  * Many compute_dynamic chains (green_class_compute_dynamic.f90:191-334) at
  * once, as compute_greenAA issues them for every sector, particle/hole part,
  * eigenstate and orbital combination (green_class_computeAA.f90:105-126).
- * mode 0: one persistent launch over a work queue (largest chains first, one
- * thread block per chain, launch shape autotuned once per problem class and
- * cached on the context); mode 1: one grid per Lanczos step, chain after chain.
+ * mode 0: one persistent launch over a work queue (largest chains first, a
+ * cluster of 1 to 16 thread blocks per chain, launch shape autotuned once per
+ * problem class and cached on the context); mode 1: one grid per Lanczos step, chain after chain.
  * G_out[out][w] (interleaved re/im, nout x nw) accumulates weight * dyn. */
 typedef struct edk_chain {
     edk_h *target;               /* Hamiltonian of the sector start_dev lives in */
