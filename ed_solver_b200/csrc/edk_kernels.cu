@@ -30,7 +30,7 @@
 // (lanc_opt, Lanczos_plain.h:66-173, without its separate orthogonalise and
 // normalise passes).  The shift keeps |s| near beta, so the rounding of the
 // stored s is not amplified by |alpha|/beta when H s is formed.
-// Reductions are deterministic: per-block partials, summed in block order by
+// Reductions are deterministic: per-block partials, summed in a fixed order by
 // the last block to finish.
 #include <cuda_runtime.h>
 #include <cstdint>
