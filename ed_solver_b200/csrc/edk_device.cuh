@@ -102,21 +102,25 @@ __device__ __forceinline__ void stage_row(T *dst, const T *src, int64_t n)
     const uintptr_t addr = reinterpret_cast<uintptr_t>(src);
     int64_t head = (int64_t)(((16u - (addr & 15u)) & 15u) / sizeof(T));
     if (head > n) head = n;
-    for (int64_t i = threadIdx.x; i < head; i += blockDim.x) dst[i] = __ldg(src + i);
+    for (int64_t i = threadIdx.x; i < head; i += blockDim.x) dst[i] = src[i];
     const int64_t nv = (n - head) / V;
     const int4 *sv = reinterpret_cast<const int4 *>(src + head);
     for (int64_t i = threadIdx.x; i < nv; i += blockDim.x) {
-        int4 q = __ldg(sv + i);
+        int4 q = sv[i];
         T tmp[V];
         memcpy(tmp, &q, 16);
 #pragma unroll
         for (int v = 0; v < V; ++v) dst[head + i * V + v] = tmp[v];
     }
-    for (int64_t i = head + nv * V + threadIdx.x; i < n; i += blockDim.x) dst[i] = __ldg(src + i);
+    for (int64_t i = head + nv * V + threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
 }
 
 
 // L2 eviction-priority policies (createpolicy) and loads/stores carrying them.
+// The loads are of Krylov vectors, which an earlier kernel of the chain wrote:
+// they keep off the read-only path (ld.global.nc, __ldg), which wants data that
+// nothing writes while the kernel lives, and a chained kernel lives from before
+// the end of the one that writes its vectors (edk_launch.cuh).
 __device__ __forceinline__ uint64_t l2_keep()
 {
     uint64_t p;
@@ -132,13 +136,13 @@ __device__ __forceinline__ uint64_t l2_stream()
 __device__ __forceinline__ float2 ld2(const float *p, uint64_t pol)
 {
     float2 v;
-    asm volatile("ld.global.nc.L2::cache_hint.v2.f32 {%0,%1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(p), "l"(pol));
+    asm volatile("ld.global.L2::cache_hint.v2.f32 {%0,%1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(p), "l"(pol));
     return v;
 }
 __device__ __forceinline__ double2 ld2(const double *p, uint64_t pol)
 {
     double2 v;
-    asm volatile("ld.global.nc.L2::cache_hint.v2.f64 {%0,%1}, [%2], %3;" : "=d"(v.x), "=d"(v.y) : "l"(p), "l"(pol));
+    asm volatile("ld.global.L2::cache_hint.v2.f64 {%0,%1}, [%2], %3;" : "=d"(v.x), "=d"(v.y) : "l"(p), "l"(pol));
     return v;
 }
 __device__ __forceinline__ void st2(float *p, float a, float b, uint64_t pol)
@@ -152,7 +156,7 @@ __device__ __forceinline__ void st2(double *p, double a, double b, uint64_t pol)
 __device__ __forceinline__ float4 ld4(const float *p, uint64_t pol)
 {
     float4 v;
-    asm volatile("ld.global.nc.L2::cache_hint.v4.f32 {%0,%1,%2,%3}, [%4], %5;"
+    asm volatile("ld.global.L2::cache_hint.v4.f32 {%0,%1,%2,%3}, [%4], %5;"
                  : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(pol));
     return v;
 }
@@ -164,13 +168,13 @@ __device__ __forceinline__ void st4(float *p, float a, float b, float c, float d
 __device__ __forceinline__ float ld1(const float *p, uint64_t pol)
 {
     float v;
-    asm volatile("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
+    asm volatile("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
     return v;
 }
 __device__ __forceinline__ double ld1(const double *p, uint64_t pol)
 {
     double v;
-    asm volatile("ld.global.nc.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
+    asm volatile("ld.global.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
     return v;
 }
 __device__ __forceinline__ void st1(float *p, float a, uint64_t pol)
@@ -180,6 +184,27 @@ __device__ __forceinline__ void st1(float *p, float a, uint64_t pol)
 __device__ __forceinline__ void st1(double *p, double a, uint64_t pol)
 {
     asm volatile("st.global.L2::cache_hint.f64 [%0], %1, %2;" :: "l"(p), "d"(a), "l"(pol) : "memory");
+}
+// The same through the read-only path, for kernels that are launched plainly (the
+// grid before them has ended) and vectors that they do not write themselves.
+__device__ __forceinline__ float ldr1(const float *p, uint64_t pol)
+{
+    float v;
+    asm volatile("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
+    return v;
+}
+__device__ __forceinline__ float2 ldr2(const float *p, uint64_t pol)
+{
+    float2 v;
+    asm volatile("ld.global.nc.L2::cache_hint.v2.f32 {%0,%1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(p), "l"(pol));
+    return v;
+}
+__device__ __forceinline__ float4 ldr4(const float *p, uint64_t pol)
+{
+    float4 v;
+    asm volatile("ld.global.nc.L2::cache_hint.v4.f32 {%0,%1,%2,%3}, [%4], %5;"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(pol));
+    return v;
 }
 __device__ __forceinline__ void prefetch_l2(const void *p)
 {

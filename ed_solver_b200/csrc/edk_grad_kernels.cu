@@ -51,8 +51,7 @@ __global__ void dots_kernel(int64_t n, const double *x0, const double *y0, const
 // in a fixed order into its own slot, blocks write per-parameter partials and
 // the last block sums them, a warp per parameter, in a fixed order.
 template <bool STAGE>
-__global__ void __launch_bounds__(512, 1) bilinear_kernel(int dup, int ddn, const double *__restrict__ a,
-                                                          const double *__restrict__ b,
+__global__ void __launch_bounds__(512, 1) bilinear_kernel(int dup, int ddn, const double *a, const double *b,
                                                           const uint32_t *__restrict__ st_up,
                                                           const uint32_t *__restrict__ st_dn, int np,
                                                           const ParamDev *__restrict__ P, double *partials,

@@ -70,7 +70,7 @@ __device__ __forceinline__ double hund_terms(const HamDev &H, const T *x, int64_
             const int32_t pd = H.dn.move[ido * H.nmove + md];
             if (pu == 0 || pd == 0) continue;
             const int64_t ju = (pu > 0 ? pu : -pu) - 1, jd = (pd > 0 ? pd : -pd) - 1;
-            const double t = fmul((double)__ldg(x + ju + jd * H.dup), jj[s1 * nc + s2]);
+            const double t = fmul((double)x[ju + jd * H.dup], jj[s1 * nc + s2]);
             acc = ((pu > 0) == (pd > 0)) ? fadd(acc, t) : fsub(acc, t);
         }
     }
@@ -85,7 +85,7 @@ __device__ __forceinline__ double hund_terms(const HamDev &H, const T *x, int64_
             const int32_t pd = H.dn.move[ido * H.nmove + m];
             if (pu == 0 || pd == 0) continue;
             const int64_t ju = (pu > 0 ? pu : -pu) - 1, jd = (pd > 0 ? pd : -pd) - 1;
-            const double t = fmul((double)__ldg(x + ju + jd * H.dup), jj[s1 * nc + s2]);
+            const double t = fmul((double)x[ju + jd * H.dup], jj[s1 * nc + s2]);
             acc = ((pu > 0) == (pd > 0)) ? fadd(acc, t) : fsub(acc, t);
         }
     }
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(512, 1) row_kernel(const HamDev H, const RowAr
     __shared__ double s_hd[R][KB];
     T *xs = reinterpret_cast<T *>(smem_raw);
     const int64_t dup = H.dup, ddn = H.ddn;
-    const T *__restrict__ x = static_cast<const T *>(a.x);
+    const T *x = static_cast<const T *>(a.x);
 
     chain_next();
     if (PACKED) {
@@ -196,10 +196,10 @@ __global__ void __launch_bounds__(512, 1) row_kernel(const HamDev H, const RowAr
                 for (int r = 0; r < R; ++r)
 #pragma unroll
                     for (int f = 0; f < KB; ++f)
-                        xd[r][f] = (row[r] >= 0 && f < s_nd[r]) ? __ldg(x + (int64_t)s_jd[r][f] * dup + c) : T(0);
+                        xd[r][f] = (row[r] >= 0 && f < s_nd[r]) ? x[(int64_t)s_jd[r][f] * dup + c] : T(0);
 #pragma unroll
                 for (int r = 0; r < R; ++r)
-                    xo[r] = row[r] < 0 ? T(0) : (STAGE ? xs[(size_t)r * dup + c] : __ldg(x + (int64_t)row[r] * dup + c));
+                    xo[r] = row[r] < 0 ? T(0) : (STAGE ? xs[(size_t)r * dup + c] : x[(int64_t)row[r] * dup + c]);
                 // ---- accumulate in the reference order ----
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(512, 1) row_kernel(const HamDev H, const RowAr
                     const double h = PACKED ? pal_s[ent[k] >> 24] : hv[k];
 #pragma unroll
                     for (int r = 0; r < R; ++r) {
-                        const T xj = STAGE ? xs[(size_t)r * dup + j] : __ldg(x + (int64_t)row[r] * dup + j);
+                        const T xj = STAGE ? xs[(size_t)r * dup + j] : x[(int64_t)row[r] * dup + j];
                         acc[r] = hmadd<T>(acc[r], h, xj);
                     }
                 }
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(512, 1) row_kernel(const HamDev H, const RowAr
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
                     if (row[r] < 0) { acc[r] = 0.0; xo[r] = T(0); continue; }
-                    xo[r] = STAGE ? xs[(size_t)r * dup + c] : __ldg(x + (int64_t)row[r] * dup + c);
+                    xo[r] = STAGE ? xs[(size_t)r * dup + c] : x[(int64_t)row[r] * dup + c];
                     const int cfg = cu * H.ncfg + cd[r];
                     const int o0 = H.int_off[cfg], o1 = H.int_off[cfg + 1];
                     double ac = 0.0;
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(512, 1) row_kernel(const HamDev H, const RowAr
 #pragma unroll
                     for (int r = 0; r < R; ++r) {
                         if (row[r] < 0) continue;
-                        const T xj = STAGE ? xs[(size_t)r * dup + j] : __ldg(x + (int64_t)row[r] * dup + j);
+                        const T xj = STAGE ? xs[(size_t)r * dup + j] : x[(int64_t)row[r] * dup + j];
                         acc[r] = hmadd<T>(acc[r], h, xj);
                     }
                 }
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(512, 1) row_kernel(const HamDev H, const RowAr
                     const int f0 = H.dn.ptr[row[r]], f1 = H.dn.ptr[row[r] + 1];
                     for (int f = f0; f < f1; ++f) {
                         const int64_t jd = H.dn.tgt[f];
-                        acc[r] = hmadd<T>(acc[r], dnv[f], __ldg(x + jd * dup + c));
+                        acc[r] = hmadd<T>(acc[r], dnv[f], x[jd * dup + c]);
                     }
                     if (H.hund) acc[r] = hund_terms<T>(H, x, c, row[r], cu, cd[r], acc[r]);
                 }

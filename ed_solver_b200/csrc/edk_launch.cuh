@@ -19,7 +19,9 @@ namespace edk {
 
 // Everything the kernels before this one wrote is visible after it, and they
 // have ended.  Every block of a kernel launched with launch_chained calls it,
-// before it reads or writes anything another kernel may write or read.
+// before it reads or writes anything another kernel may write or read.  What another
+// kernel of the chain wrote is read with ordinary loads or ld.cg, not through the
+// read-only path and not through const __restrict__ pointers.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // The next kernel may start its blocks once all of this one's have come here.
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

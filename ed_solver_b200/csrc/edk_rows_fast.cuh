@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(NTHR, MINB) row_fast_kernel(const HamDev H, co
     T *xs = reinterpret_cast<T *>(smem_raw);
     const int dup = (int)H.dup;
     const int64_t ddn = H.ddn;
-    const T *__restrict__ x = static_cast<const T *>(a.x);
+    const T *x = static_cast<const T *>(a.x);
 
     chain_next();
     {
@@ -134,17 +134,17 @@ __global__ void __launch_bounds__(NTHR, MINB) row_fast_kernel(const HamDev H, co
                 const uintptr_t addr = reinterpret_cast<uintptr_t>(src);
                 int head = (int)(((16u - (addr & 15u)) & 15u) / sizeof(T));
                 if (head > dup) head = dup;
-                for (int i = threadIdx.x; i < head; i += blockDim.x) xs[i * R + r] = __ldg(src + i);
+                for (int i = threadIdx.x; i < head; i += blockDim.x) xs[i * R + r] = src[i];
                 const int nv = (dup - head) / V;
                 const int4 *sv = reinterpret_cast<const int4 *>(src + head);
                 for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-                    const int4 q = __ldg(sv + i);
+                    const int4 q = sv[i];
                     T tmp[V];
                     memcpy(tmp, &q, 16);
 #pragma unroll
                     for (int v = 0; v < V; ++v) xs[(head + i * V + v) * R + r] = tmp[v];
                 }
-                for (int i = head + nv * V + threadIdx.x; i < dup; i += blockDim.x) xs[i * R + r] = __ldg(src + i);
+                for (int i = head + nv * V + threadIdx.x; i < dup; i += blockDim.x) xs[i * R + r] = src[i];
             }
         }
         __syncthreads();

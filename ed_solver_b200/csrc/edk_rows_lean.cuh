@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(NT, MINB) row_lean_kernel(const HamDev H, cons
             const float *x0 = x + (int64_t)d0 * dup, *x1 = x + (int64_t)d1 * dup;
 #pragma unroll 4
             for (int u = 2 * tid; u < dup; u += 2 * NT) {
-                const float2 p = ld2(x0 + u, keep), q = ld2(x1 + u, keep);
+                const float2 p = ldr2(x0 + u, keep), q = ldr2(x1 + u, keep);
                 *reinterpret_cast<float4 *>(xs2 + u) = make_float4(p.x, q.x, p.y, q.y);
             }
         }
@@ -137,12 +137,12 @@ __global__ void __launch_bounds__(NT, MINB) row_lean_kernel(const HamDev H, cons
         auto load = [&](int c, Ld &L) {
 #pragma unroll
             for (int f = 0; f < KMD; ++f) {
-                L.xd[0][f] = ld2(x + nofs[0][f] + c, keep);
-                L.xd[1][f] = ld2(x + nofs[1][f] + c, keep);
+                L.xd[0][f] = ldr2(x + nofs[0][f] + c, keep);
+                L.xd[1][f] = ldr2(x + nofs[1][f] + c, keep);
             }
             if (mode == kModeStep) {
-                L.vk[0] = ld2(vkp + ib0 + c, stream);
-                L.vk[1] = ld2(vkp + ib1 + c, stream);
+                L.vk[0] = ldr2(vkp + ib0 + c, stream);
+                L.vk[1] = ldr2(vkp + ib1 + c, stream);
                 if (vmp) {
                     L.vm[0] = ld2(vmp + ib0 + c, stream);
                     L.vm[1] = ld2(vmp + ib1 + c, stream);

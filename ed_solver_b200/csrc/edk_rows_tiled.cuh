@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(NT, MINB) up_pass_kernel(const HamDev H, const
             float2 *dst = xs2 + (size_t)p * dup;
 #pragma unroll 4
             for (int u = 2 * tid; u < dup; u += 2 * NT) {
-                const float2 a0 = ld2(x0 + u, keep), a1 = ld2(x1 + u, keep);
+                const float2 a0 = ldr2(x0 + u, keep), a1 = ldr2(x1 + u, keep);
                 *reinterpret_cast<float4 *>(dst + u) = make_float4(a0.x, a1.x, a0.y, a1.y);
             }
         }
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(NT, 1) up_pass_quad_kernel(const HamDev H, con
             const float *x2 = x + (int64_t)d[2] * dup, *x3 = x + (int64_t)d[3] * dup;
 #pragma unroll 2
             for (int u = tid; u < dup; u += NT)
-                xs4[u] = make_float4(ld1(x0 + u, keep), ld1(x1 + u, keep), ld1(x2 + u, keep), ld1(x3 + u, keep));
+                xs4[u] = make_float4(ldr1(x0 + u, keep), ldr1(x1 + u, keep), ldr1(x2 + u, keep), ldr1(x3 + u, keep));
         }
         __syncthreads();
         int cd[R];
@@ -319,12 +319,12 @@ __global__ void __launch_bounds__(256, 4) down_pass_kernel(const HamDev H, const
             // every global load of the element pair first
             float2 xd[KMD];
 #pragma unroll
-            for (int f = 0; f < KMD; ++f) xd[f] = ld2(x + s_nofs[r][f] + c, keep);
-            const float2 own = ld2(x + i, keep);
-            const float2 yv = ld2(y1 + i, stream);
+            for (int f = 0; f < KMD; ++f) xd[f] = ldr2(x + s_nofs[r][f] + c, keep);
+            const float2 own = ldr2(x + i, keep);
+            const float2 yv = ldr2(y1 + i, stream);
             float2 vk2 = make_float2(0.f, 0.f), vm2 = make_float2(0.f, 0.f);
             if (mode == kModeStep) {
-                vk2 = ld2(vkp + i, stream);
+                vk2 = ldr2(vkp + i, stream);
                 if (vmp) vm2 = ld2(vmp + i, stream);
             }
             const int nd = s_nd[r];
@@ -434,12 +434,12 @@ __global__ void __launch_bounds__(256, 3) down_pass4_kernel(const HamDev H, cons
             // every global load of the four elements first
             float4 xd[KMD];
 #pragma unroll
-            for (int f = 0; f < KMD; ++f) xd[f] = ld4(x + s_nofs[r][f] + c, keep);
-            const float4 own = ld4(x + i, keep);
-            const float4 yv = ld4(y1 + i, stream);
+            for (int f = 0; f < KMD; ++f) xd[f] = ldr4(x + s_nofs[r][f] + c, keep);
+            const float4 own = ldr4(x + i, keep);
+            const float4 yv = ldr4(y1 + i, stream);
             float4 vk4 = make_float4(0.f, 0.f, 0.f, 0.f), vm4 = make_float4(0.f, 0.f, 0.f, 0.f);
             if (mode == kModeStep) {
-                vk4 = ld4(vkp + i, stream);
+                vk4 = ldr4(vkp + i, stream);
                 if (vmp) vm4 = ld4(vmp + i, stream);
             }
             const int nd = s_nd[r];

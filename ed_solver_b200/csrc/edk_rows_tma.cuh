@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
     T *rowbuf = reinterpret_cast<T *>(smem_raw);   // [2][R][slot]
     const int dup = (int)H.dup;
     const int64_t ddn = H.ddn;
-    const T *__restrict__ x = static_cast<const T *>(a.x);
+    const T *x = static_cast<const T *>(a.x);
     const int tid = threadIdx.x;
 
     chain_next();
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
                 const int nhead = c16, ntail = dup - ce16;
                 for (int i = tid - kRagged; i < nhead + ntail; i += nr) {
                     const int c = i < nhead ? i : ce16 + (i - nhead);
-                    dst[c] = __ldg(src + c);
+                    dst[c] = src[c];
                 }
             }
         }
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(NTHR, MINB) row_tma_kernel(const HamDev H, con
                 const int ju = (hp[e] > 0 ? hp[e] : -hp[e]) - 1;
 #pragma unroll
                 for (int r = 0; r < R; ++r)
-                    hx[r][e] = hp[e] && s_hofs[b][r] >= 0 ? __ldg(x + s_hofs[b][r] + ju) : T(0);
+                    hx[r][e] = hp[e] && s_hofs[b][r] >= 0 ? x[s_hofs[b][r] + ju] : T(0);
             }
         }
         // density terms, diagonal (FP64)

@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(NTMAX, MINB) sz_row_kernel(const SzDev S, cons
     StepScalars sc;
     if (!step_scalars(a, ks, sc)) return;
 
-    const T *__restrict__ x = static_cast<const T *>(a.x);
+    const T *x = static_cast<const T *>(a.x);
     const int ns = S.ns, nb = S.nb, nc = S.nc, nrun = S.nrun, NT = blockDim.x, lane = threadIdx.x & 31;
     const uint32_t cm = (1u << nc) - 1u;
     const uint32_t nlow = 1u << ns;
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(NTMAX, MINB) sz_row_kernel(const SzDev S, cons
         const uint32_t *__restrict__ ell = S.ell + c0;
         const uint32_t *__restrict__ pair = S.pair + c0;
         const double *__restrict__ pdiag = S.pdiag + ((size_t)hcfg << ns) + c0;
-        const T *__restrict__ xrow = x + base;
+        const T *xrow = x + base;
         const uint32_t *__restrict__ kell = S.kell + k * nrun;
         // a warp owns 64 adjacent columns, two per lane: c and c + step (step = 32 where the
         // warp's columns all exist, so that it folds into the loads' immediate offsets;
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(NTMAX, MINB) sz_row_kernel(const SzDev S, cons
             const int c = FULL ? cw + lane : min(cw + lane, len - 1);
             const int step = FULL ? 32 : min(cw + 32 + lane, len - 1) - c;
             const uint32_t l[2] = {(uint32_t)S.low_states[c0 + c], (uint32_t)S.low_states[c0 + c + step]};
-            const T xo[2] = {STAGE ? xs[c] : __ldg(xrow + c), STAGE ? xs[c + step] : __ldg(xrow + c + step)};
+            const T xo[2] = {STAGE ? xs[c] : xrow[c], STAGE ? xs[c + step] : xrow[c + step]};
             double acc[2];
 #pragma unroll
             for (int e = 0; e < 2; ++e) acc[e] = fmul(qs[((l[e] >> nb) & cm) | (hcfg << nc)], (double)xo[e]);
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(NTMAX, MINB) sz_row_kernel(const SzDev S, cons
                         for (int e = 0; e < 2; ++e) {
                             const double g = *reinterpret_cast<const double *>(h2b + (u[e] >> 16));
                             const uint32_t col = u[e] & 0xFFFFu;
-                            const T xv = STAGE ? xs[col] : __ldg(xrow + col);
+                            const T xv = STAGE ? xs[col] : xrow[col];
                             if (u[e] < pad) acc[e] = hmadd<T>(acc[e], g, xv);
                         }
                     }
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(NTMAX, MINB) sz_row_kernel(const SzDev S, cons
 #pragma unroll 4
                     for (int q = e0; q < e1; ++q) {
                         const T *p = reinterpret_cast<const T *>(xc + rt[q].xoff);
-                        const T x0 = __ldg(p), x1 = __ldg(p + step);
+                        const T x0 = p[0], x1 = p[step];
                         const double g = hv[q];
                         acc[0] = hmadd<T>(acc[0], g, x0);
                         acc[1] = hmadd<T>(acc[1], g, x1);
@@ -254,8 +254,8 @@ __global__ void __launch_bounds__(NTMAX, MINB) sz_row_kernel(const SzDev S, cons
                             for (int e = 0; e < 2; ++e) {
                                 ta[e] ^= oa.want & 0x20000u;
                                 tb[e] ^= ob.want & 0x20000u;
-                                va[e] = __ldg(ra + (ta[e] & 0x20000u ? 0u : ta[e] & 0xFFFFu));
-                                vb[e] = __ldg(rb + (tb[e] & 0x20000u ? 0u : tb[e] & 0xFFFFu));
+                                va[e] = ra[ta[e] & 0x20000u ? 0u : ta[e] & 0xFFFFu];
+                                vb[e] = rb[tb[e] & 0x20000u ? 0u : tb[e] & 0xFFFFu];
                             }
                             const double ga = hv[qa], gb = hv[qb];
 #pragma unroll
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) sz_wide_kernel(const SzDev S, c
     StepScalars sc;
     if (!step_scalars(a, ks, sc)) return;
 
-    const T *__restrict__ x = static_cast<const T *>(a.x);
+    const T *x = static_cast<const T *>(a.x);
     const int ns = S.ns, nb = S.nb, nc = S.nc, nrun = S.nrun;
     const uint32_t cm = (1u << nc) - 1u, nlow = 1u << ns;
     const unsigned char *h2b = reinterpret_cast<const unsigned char *>(h2);
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) sz_wide_kernel(const SzDev S, c
                         const T *p = reinterpret_cast<const T *>(xc + rt[q].xoff);
                         T v[NS];
 #pragma unroll
-                        for (int i = 0; i < NS; ++i) v[i] = __ldg(p + off(i));
+                        for (int i = 0; i < NS; ++i) v[i] = p[off(i)];
                         const double g = hv[q];
 #pragma unroll
                         for (int i = 0; i < NS; ++i) acc[i] = hmadd<T>(acc[i], g, v[i]);
@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(kSzBlock) sz_row_simple_kernel(const SzDev S, 
     if (!step_scalars(a, ks, sc)) return;
     __syncthreads();
 
-    const T *__restrict__ x = static_cast<const T *>(a.x);
+    const T *x = static_cast<const T *>(a.x);
     const int ns = S.ns, nb = S.nb, nc = S.nc, nterm = S.nterm, ndiag = S.ndiag;
     const uint32_t lowmask = (1u << ns) - 1u, cm = (1u << nc) - 1u;
     const uint32_t *__restrict__ off_h = S.sec.off_h;
@@ -553,7 +553,7 @@ __global__ void __launch_bounds__(kSzBlock) sz_row_simple_kernel(const SzDev S, 
                 const uint32_t s2t = s ^ src ^ tgt;
                 const int64_t j = (int64_t)off_h[s2t >> ns] + rank_low[s2t & lowmask];
                 const double hv = (__popc(s & ts[t].btw) & 1) ? -ts[t].h : ts[t].h;
-                acc = hmadd<T>(acc, hv, __ldg(x + j));
+                acc = hmadd<T>(acc, hv, x[j]);
             }
             row_epilogue<T>(a, sc, i, acc, xo, s0, s1, s2);
         }
