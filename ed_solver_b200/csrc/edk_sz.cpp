@@ -423,7 +423,9 @@ int sz_create(const edk_model_sz *m, int npart, cudaStream_t st, SzHost **out, s
     d.pdiag = z->pdiag.as<double>();
     d.pair = z->pair.as<uint32_t>();
     d.kell = z->kell.as<uint32_t>();
-    if (nrow > 0 && (e = launch_sz_pair(d, nrow, z->pair.as<uint32_t>(), st)) != cudaSuccess) {
+    // waited for, like the uploads: the sector may be used on any stream once it exists
+    if (nrow > 0 && ((e = launch_sz_pair(d, nrow, z->pair.as<uint32_t>(), st)) != cudaSuccess ||
+                     (e = cudaStreamSynchronize(st)) != cudaSuccess)) {
         *err = std::string("Nambu sector tables: ") + cudaGetErrorString(e);
         return EDK_ERR_CUDA;
     }
