@@ -505,7 +505,8 @@ static cudaError_t launch_gs_batch_t(const HamDev *hams, const GsItem *items, in
 {
     auto k = gs_batch_kernel<T, R>;
     const size_t smem = (((size_t)R * maxdup * sizeof(T) + 15) & ~(size_t)15) + (size_t)2 * nmax * sizeof(double);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int per_sm = 0;
+    cudaError_t e = kernel_fit(reinterpret_cast<const void *>(k), 512, smem, &per_sm);
     if (e != cudaSuccess) return e;
     k<<<grid, 512, smem, st>>>(hams, items, nitems, queue, static_cast<T *>(work), maxdim, (int)maxdup, nmax, tab,
                                cutoff, every, pass);

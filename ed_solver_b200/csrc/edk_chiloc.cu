@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "../../include/edk.h"
+#include "edk_launch.cuh"
 
 namespace {
 
@@ -931,8 +932,9 @@ static int chiloc_factored(edk_ctx *ctx, const ChiArgs &A_in, const std::vector<
     }
     grid = std::min(grid, nitem);
     cudaError_t e = cudaMemcpyAsync(d, h, nIn * 8, cudaMemcpyHostToDevice, st);
+    int per_sm = 0;      // allows the shared memory, for every size: the limit is the process's
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(chi_factored_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = edk::kernel_fit(reinterpret_cast<const void *>(chi_factored_kernel), kChiBlock, smem, &per_sm);
     if (e == cudaSuccess) {
         A.E = d;
         A.C = d + nE;
@@ -1053,8 +1055,10 @@ int edk_chiloc(edk_ctx *ctx, int32_t op_mask, double beta, double Z, double gs_e
         const int use_jk = smem_jk <= cap ? 1 : 0;
         const size_t smem = use_jk ? smem_jk : smem_1d;
         const bool split = smem <= cap;
-        if (split && smem > 48 * 1024)
-            cudaFuncSetAttribute(chi_terms_hoisted_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        int per_sm = 0;
+        if (split && (e = edk::kernel_fit(reinterpret_cast<const void *>(chi_terms_hoisted_kernel), kChiBlock, smem,
+                                          &per_sm)) != cudaSuccess)
+            return edk_internal_fail(ctx, EDK_ERR_CUDA, cudaGetErrorString(e));
         // grid.z is limited to 65535: frequency triples in chunks
         for (int f0 = 0; f0 < nf; f0 += 65535) {
             ChiArgs Ac = A;

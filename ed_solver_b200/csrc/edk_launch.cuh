@@ -27,7 +27,9 @@ __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Allows `kernel` the dynamic shared memory `smem` and gives the blocks of
-// `threads` threads that an SM holds.
+// `threads` threads that an SM holds.  The limit belongs to the process: it is set
+// to all the kernel can have, never to one call's need, which another thread's
+// smaller call could lower between this one's setting and its launch.
 cudaError_t kernel_fit(const void *kernel, int threads, size_t smem, int *per_sm);
 
 template <typename... K, typename... A>

@@ -260,10 +260,8 @@ cudaError_t launch_lean_t(const HamDev &H, const RowArgs &a, int num_sms, cudaSt
 {
     auto k = a.mode == kModeStep ? row_lean_kernel<KS, KMD, NT, MINB, true> : row_lean_kernel<KS, KMD, NT, MINB, false>;
     const size_t smem = lean_smem_bytes(H.dup);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, NT, smem);
+    cudaError_t e = kernel_fit(reinterpret_cast<const void *>(k), NT, smem, &per_sm);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     const int64_t groups = (H.ddn + 1) / 2;

@@ -533,10 +533,8 @@ cudaError_t launch_tiled_t(const HamDev &H, const RowArgs &a, int num_sms, int v
                  : two  ? (sp ? up_pass_kernel<KS, 2, 512, 1, true> : up_pass_kernel<KS, 2, 512, 1, false>)
                         : (sp ? up_pass_kernel<KS, 1, 512, 2, true> : up_pass_kernel<KS, 1, 512, 2, false>);
         const size_t smem = two ? 2 * pair : pair;
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
         int per_sm = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, nt, smem);
+        cudaError_t e = kernel_fit(reinterpret_cast<const void *>(k), nt, smem, &per_sm);
         if (e != cudaSuccess) return e;
         if (per_sm < 1) return cudaErrorInvalidConfiguration;
         const int64_t groups = (H.ddn + (two ? 3 : 1)) / (two ? 4 : 2);
@@ -549,7 +547,7 @@ cudaError_t launch_tiled_t(const HamDev &H, const RowArgs &a, int num_sms, int v
     auto k2 = four ? (a.mode == kModeStep ? down_pass4_kernel<KMD, true> : down_pass4_kernel<KMD, false>)
                    : (a.mode == kModeStep ? down_pass_kernel<KMD, true> : down_pass_kernel<KMD, false>);
     int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k2, 256, 0);
+    cudaError_t e = kernel_fit(reinterpret_cast<const void *>(k2), 256, 0, &per_sm);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     k2<<<num_sms * per_sm, 256, 0, st>>>(H, a, y1);
