@@ -874,6 +874,7 @@ int edk_chiloc_set_kernel(int plain)
 int edk_internal_fail(edk_ctx *ctx, int code, const char *msg);
 void *edk_internal_scratch(edk_ctx *ctx, int slot, size_t bytes);
 void edk_internal_scratch_done(edk_ctx *ctx);
+void edk_internal_scratch_free(edk_ctx *ctx);
 int edk_internal_num_sms(const edk_ctx *ctx);
 void edk_internal_add_launches(edk_ctx *ctx, int64_t n);
 void edk_internal_count(edk_ctx *ctx, int64_t h2d, int64_t d2h);
@@ -951,8 +952,8 @@ static int chiloc_factored(edk_ctx *ctx, const ChiArgs &A_in, const std::vector<
             e = cudaMemcpyAsync(o, d + nIn + (size_t)op * 2 * A.nf, sizeof(double) * 2 * A.nf, cudaMemcpyDeviceToHost,
                                 st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return edk_internal_fail(ctx, EDK_ERR_CUDA, cudaGetErrorString(e));
     edk_internal_scratch_done(ctx);
+    if (e != cudaSuccess) return edk_internal_fail(ctx, EDK_ERR_CUDA, cudaGetErrorString(e));
     edk_internal_count(ctx, (int64_t)(nIn - nT) * 8, (int64_t)A.nf * 16 * ((out1 ? 1 : 0) + (out2 ? 1 : 0)));
     return EDK_OK;
 }
@@ -1024,6 +1025,7 @@ int edk_chiloc(edk_ctx *ctx, int32_t op_mask, double beta, double Z, double gs_e
         const int rc = chiloc_factored(ctx, A, terms, E, C, boltz, w_host, (op_mask & 1) ? pdndn_host : nullptr,
                                        (op_mask & 2) ? pupdn_host : nullptr);
         if (rc != kNotFactored) return rc;
+        edk_internal_scratch_free(ctx);      // the kernels below may need that memory
     }
     DevMem dE, dC, dT, dW, dP, dB, dO;
     cudaError_t e;

@@ -1071,6 +1071,12 @@ void edk_internal_scratch_done(edk_ctx *ctx)
         if (b.bytes > (size_t)256 << 20) b.release();
 }
 
+// All of them, for a call that goes on without.
+void edk_internal_scratch_free(edk_ctx *ctx)
+{
+    for (DevBuf &b : ctx->scratch) b.release();
+}
+
 int edk_internal_fail(edk_ctx *ctx, int code, const char *msg) { return ctx->fail(code, "%s", msg); }
 
 edk_ctx *edk_internal_h_ctx(edk_h *h) { return h->ctx; }
@@ -1174,7 +1180,7 @@ int edk_ctx_trim(edk_ctx *ctx)
     if (!ctx) return EDK_ERR_INVALID;
     int rc = ctx->cuda(cudaStreamSynchronize(ctx->stream), "sync");
     if (rc) return rc;
-    for (DevBuf &b : ctx->scratch) b.release();
+    edk_internal_scratch_free(ctx);
     if (!ctx->basis_pool) return EDK_OK;
     return ctx->cuda(cudaMemPoolTrimTo(ctx->basis_pool, 0), "cudaMemPoolTrimTo");
 }
