@@ -511,6 +511,10 @@ int fast_shape_for(edk_h *h, int dtype, const RowArgs &a, bool aligned, FastShap
     const int n = fast_shapes(h->H, eb, c->num_sms, cand, kMaxShapes, a.sum32);
     if (n == 0) return c->fail(EDK_ERR_INVALID, "fast row kernel: no launch shape");
     out = cand[0];
+    // inside a caller's capture nothing can be timed: a later call does it
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &capture) != cudaSuccess) (void)cudaGetLastError();
+    if (capture != cudaStreamCaptureStatusNone) return EDK_OK;
     if (c->kernel_path != 0 || n == 1 || !a.x || !a.y) {
         if (n == 1 || c->kernel_path != 0) { h->fast_shape[slot] = out; h->fast_tuned[slot] = true; }
         return EDK_OK;
