@@ -558,7 +558,7 @@ int edk_grad_green(edk_h *h, const void *psi_dev, double e0, int32_t nchain, con
             }
             if (stats) {
                 stats->cg_iterations = cg.it;
-                stats->cg_residual = std::sqrt(cg.rr / cg.rr0);
+                stats->cg_residual = cg.it > 0 ? std::sqrt(cg.rr / cg.rr0) : 0.0;   // rr0 may be 0
             }
             if ((rc = ops_bilinear(o, x, psi, tb.data()))) return rc;
             for (int q = 0; q < np; ++q) grad[q] -= tb[q];
