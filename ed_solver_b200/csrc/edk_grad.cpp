@@ -286,6 +286,10 @@ struct Vec {
     }
 };
 
+// Elements of one array of the continued fraction (64 MB): with the frequencies all
+// at once a call's memory would grow with steps times frequencies.
+constexpr int kCfElements = 1 << 22;
+
 // Forward Lanczos of phi (K steps or until breakdown) keeping checkpoints, the
 // continued fraction with its vector-Jacobian product, then the reverse sweep, all
 // queued on the stream: every coefficient stays on the device (GradScalars), and
@@ -309,19 +313,18 @@ int chain_vjp(edk_h *ht, Ops &o, const double *phi, int K, double e0, double ph,
     const int m = std::max(2, (int)std::ceil(std::sqrt(2.0 * K)));
     const int nseg = (K + m - 1) / m;
     // scalars (K + 2 each), theta, and the continued fraction's buffers
+    // the latter for at most kCfElements / K frequencies at a time
+    const int nwc = std::min(nw, std::max(32, kCfElements / K));
     const size_t ks = (size_t)K + 2, nsc = 4 * ks + 8 + o.np;
-    DBuf sc(sizeof(double) * nsc, o.ctx), cf(sizeof(double) * ((size_t)nw * (4 * (size_t)K + 9)), o.ctx);
+    DBuf sc(sizeof(double) * nsc, o.ctx), cf(sizeof(double) * ((size_t)nwc * (4 * (size_t)K + 9)), o.ctx);
     if (!sc.p || !cf.p) return o.fail(EDK_ERR_NOMEM, "gradient scalars");
     const GradScalars S{sc.d(), sc.d() + ks, sc.d() + 2 * ks, sc.d() + 3 * ks, sc.d() + 4 * ks};
     double *theta = sc.d() + 4 * ks + 8;
-    double2 *cf_cp = reinterpret_cast<double2 *>(cf.p), *cf_u = cf_cp + (size_t)K * nw, *cf_gs = cf_u + (size_t)K * nw;
-    double *cf_in = reinterpret_cast<double *>(cf_gs + nw), *cf_G = cf_in + 3 * (size_t)nw, *cf_parts = cf_G + 2 * (size_t)nw;
-    std::vector<double> in(wn, wn + nw);
-    in.insert(in.end(), gbar, gbar + 2 * (size_t)nw);
+    double2 *cf_cp = reinterpret_cast<double2 *>(cf.p), *cf_u = cf_cp + (size_t)K * nwc, *cf_gs = cf_u + (size_t)K * nwc;
+    double *cf_in = reinterpret_cast<double *>(cf_gs + nwc), *cf_G = cf_in + 3 * (size_t)nwc,
+           *cf_parts = cf_G + 2 * (size_t)nwc;
     if ((rc = o.cuda(cudaMemsetAsync(sc.p, 0, sizeof(double) * nsc, o.st), "memset"))) return rc;
     if ((rc = o.cuda(cudaMemcpyAsync(S.be + 1, &b1, sizeof b1, cudaMemcpyHostToDevice, o.st), "h2d"))) return rc;
-    if ((rc = o.cuda(cudaMemcpyAsync(cf_in, in.data(), sizeof(double) * in.size(), cudaMemcpyHostToDevice, o.st), "h2d")))
-        return rc;
     const GradPass ps{n, o.grid, o.partials, o.counter, o.st};
     auto count = [&](cudaError_t e, const char *where, int launches = 1) {
         edk_internal_add_launches(o.ctx, launches);
@@ -364,9 +367,21 @@ int chain_vjp(edk_h *ht, Ops &o, const double *phi, int K, double e0, double ph,
     if (stats) stats->forward_steps += Keff;
     const bool has_next = be[Keff + 1] > 1e-25;
     // ---- continued fraction and its VJP ----
-    if ((rc = count(pass_cf(Keff, e0, ph, nw, cf_in, cf_in + nw, S, cf_cp, cf_u, cf_gs, cf_G, cf_parts, o.st),
-                    "gradient continued fraction", 2)))
-        return rc;
+    for (int w0 = 0; w0 < nw; w0 += nwc) {
+        const int nq = std::min(nwc, nw - w0);
+        std::vector<double> in(wn + w0, wn + w0 + nq);
+        in.insert(in.end(), gbar + 2 * (size_t)w0, gbar + 2 * (size_t)(w0 + nq));
+        if ((rc = o.cuda(cudaMemcpyAsync(cf_in, in.data(), sizeof(double) * in.size(), cudaMemcpyHostToDevice, o.st),
+                         "h2d")))
+            return rc;
+        if ((rc = count(pass_cf(Keff, e0, ph, nq, cf_in, cf_in + nq, S, cf_cp, cf_u, cf_gs, cf_G, cf_parts, o.st),
+                        "gradient continued fraction", 2)))
+            return rc;
+        if (G_out && nwc < nw &&
+            (rc = o.cuda(cudaMemcpyAsync(G_out + 2 * (size_t)w0, cf_G, sizeof(double) * 2 * nq, cudaMemcpyDeviceToHost,
+                                         o.st), "d2h")))
+            return rc;
+    }
     // ---- reverse sweep over segments, last first ----
     const int mseg = m + 2;
     std::vector<DBuf> seg(mseg);
@@ -419,7 +434,7 @@ int chain_vjp(edk_h *ht, Ops &o, const double *phi, int K, double e0, double ph,
         return rc;
     if ((rc = o.cuda(cudaMemcpyAsync(&e0bar_out, S.dot + 4, sizeof(double), cudaMemcpyDeviceToHost, o.st), "d2h")))
         return rc;
-    if (G_out && (rc = o.cuda(cudaMemcpyAsync(G_out, cf_G, sizeof(double) * 2 * nw, cudaMemcpyDeviceToHost, o.st), "d2h")))
+    if (G_out && nwc == nw && (rc = o.cuda(cudaMemcpyAsync(G_out, cf_G, sizeof(double) * 2 * nw, cudaMemcpyDeviceToHost, o.st), "d2h")))
         return rc;
     if ((rc = o.cuda(cudaStreamSynchronize(o.st), "sync"))) return rc;
     for (int q = 0; q < o.np; ++q) theta_bar[q] += th[q];

@@ -393,7 +393,8 @@ __global__ void cf_solve_kernel(int K, double e0, double ph, int nw, const doubl
     parts[nw + w] = (gc * ((2.0 * b1) * v)).re;             // b_1
 }
 
-// Block k < K: abar_{k+1} and bb_{k+2}; block K: E0's cotangent and bb_1.
+// Block k < K: abar_{k+1} and bb_{k+2}; block K: E0's cotangent and bb_1; added to
+// those of the frequencies before.
 __global__ void cf_reduce_kernel(int K, double ph, int nw, const double2 *u, const double2 *gs, const double *parts,
                                  GradScalars S)
 {
@@ -417,11 +418,11 @@ __global__ void cf_reduce_kernel(int K, double ph, int nw, const double2 *u, con
     block_sum<2>(s, red);
     if (threadIdx.x == 0) {
         if (k == K) {
-            S.dot[4] = s[0];
-            S.bb[1] = s[1];
+            S.dot[4] += s[0];
+            S.bb[1] += s[1];
         } else {
-            S.ab[k + 1] = s[0];
-            if (k + 1 < K) S.bb[k + 2] = s[1];
+            S.ab[k + 1] += s[0];
+            if (k + 1 < K) S.bb[k + 2] += s[1];
         }
     }
 }
