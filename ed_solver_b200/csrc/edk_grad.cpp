@@ -40,6 +40,7 @@ const uint64_t *edk_internal_h_states(const edk_h *h, int spin);
 int edk_internal_h_is_sz(const edk_h *h);
 const int32_t *edk_internal_h_rank(const edk_h *h);
 cudaMemPool_t edk_internal_pool(edk_ctx *ctx);
+int edk_internal_pinned(edk_ctx *ctx, size_t doubles, double **buf, cudaEvent_t *ev);
 }
 
 using namespace edk;
@@ -293,7 +294,7 @@ constexpr int kCfElements = 1 << 22;
 // Forward Lanczos of phi (K steps or until breakdown) keeping checkpoints, the
 // continued fraction with its vector-Jacobian product, then the reverse sweep, all
 // queued on the stream: every coefficient stays on the device (GradScalars), and
-// the host reads b_k once, to learn where the chain ends.  Adds to theta_bar
+// the host reads only b_k, to learn where the chain ends.  Adds to theta_bar
 // (target-sector parameters), writes phibar (target sector) and returns the e0bar
 // of this chain.
 //   G(z) = b_1^2 u_1 with (z - ph (T - e0)) u = e1.
@@ -339,9 +340,26 @@ int chain_vjp(edk_h *ht, Ops &o, const double *phi, int K, double e0, double ph,
         double *vkm1 = va.d(), *vk = vbuf.d(), *vnext = vc.d();
         if ((rc = o.cuda(cudaMemsetAsync(vkm1, 0, vb, o.st), "memset"))) return rc;
         if ((rc = v.lincomb(vk, false, phi, 1.0 / b1))) return rc;
+        // The host reads the b_k at each segment's start, one segment late, so that a
+        // chain that broke down is left soon and steps stay queued meanwhile.
+        double *seen = nullptr;
+        cudaEvent_t seen_ev = nullptr;
+        if (nseg > 2 && (rc = edk_internal_pinned(o.ctx, (size_t)K + 2, &seen, &seen_ev))) return rc;
         for (int k = 1; k <= K; ++k) {
             if ((k - 1) % m == 0) {
                 const int j = (k - 1) / m;
+                if (seen && j >= 2) {
+                    if ((rc = o.cuda(cudaEventSynchronize(seen_ev), "sync"))) return rc;
+                    bool broke = false;
+                    for (int q = 2; q <= k - m; ++q) broke = broke || !(seen[q] > 1e-25);
+                    if (broke) break;
+                }
+                if (seen && j >= 1 && k + m <= K) {
+                    if ((rc = o.cuda(cudaMemcpyAsync(seen, S.be, sizeof(double) * (k + 1), cudaMemcpyDeviceToHost, o.st),
+                                     "d2h")))
+                        return rc;
+                    if ((rc = o.cuda(cudaEventRecord(seen_ev, o.st), "event"))) return rc;
+                }
                 ck[2 * j] = DBuf(vb, o.ctx);
                 ck[2 * j + 1] = DBuf(vb, o.ctx);
                 if (!ck[2 * j].p || !ck[2 * j + 1].p) return o.fail(EDK_ERR_NOMEM, "gradient checkpoints");

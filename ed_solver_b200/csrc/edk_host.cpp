@@ -879,12 +879,9 @@ int fetch_tri(edk_ctx *c, int n, TriHost &t)
     return c->cuda(cudaStreamSynchronize(c->stream), "sync");
 }
 
-// Enqueue the copy of alpha_1..alpha_{n+1}, beta_0..beta_{n+1} and the flags
-// into pinned host memory and record an event after it; the host can then
-// queue more steps before waiting on the event (tri_wait).
-int tri_enqueue(edk_ctx *c, int n)
+// The context's pinned buffer, of at least `need` doubles, and its event.
+int ensure_pinned(edk_ctx *c, size_t need)
 {
-    const size_t need = (size_t)(2 * n + 8);
     if (need > c->pin_cap) {
         if (c->pin_tri) cudaFreeHost(c->pin_tri);
         c->pin_tri = nullptr;
@@ -894,14 +891,21 @@ int tri_enqueue(edk_ctx *c, int n)
         if (rc) return rc;
         c->pin_cap = cap;
     }
-    if (!c->pin_ev) {
-        int rc = c->cuda(cudaEventCreateWithFlags(&c->pin_ev, cudaEventDisableTiming), "event");
-        if (rc) return rc;
-    }
+    if (!c->pin_ev) return c->cuda(cudaEventCreateWithFlags(&c->pin_ev, cudaEventDisableTiming), "event");
+    return EDK_OK;
+}
+
+// Enqueue the copy of alpha_1..alpha_{n+1}, beta_0..beta_{n+1} and the flags
+// into pinned host memory and record an event after it; the host can then
+// queue more steps before waiting on the event (tri_wait).
+int tri_enqueue(edk_ctx *c, int n)
+{
+    int rc = ensure_pinned(c, (size_t)(2 * n + 8));
+    if (rc) return rc;
     c->d2h_bytes += (int64_t)sizeof(double) * (2 * n + 3) + 8;
     double *d = c->pin_tri, *sb = c->pin_tri + (n + 1);
     int *fl = reinterpret_cast<int *>(c->pin_tri + (2 * n + 3));
-    int rc = c->cuda(cudaMemcpyAsync(d, c->tri_diag.p, sizeof(double) * (n + 1), cudaMemcpyDeviceToHost, c->stream),
+    rc = c->cuda(cudaMemcpyAsync(d, c->tri_diag.p, sizeof(double) * (n + 1), cudaMemcpyDeviceToHost, c->stream),
                      "d2h tri");
     if (rc) return rc;
     rc = c->cuda(cudaMemcpyAsync(sb, c->tri_sub.p, sizeof(double) * (n + 2), cudaMemcpyDeviceToHost, c->stream),
@@ -1082,6 +1086,16 @@ void edk_internal_scratch_free(edk_ctx *ctx)
 }
 
 int edk_internal_fail(edk_ctx *ctx, int code, const char *msg) { return ctx->fail(code, "%s", msg); }
+
+// The context's pinned buffer (it holds until the next call that reads
+// coefficients) and the event that goes with it.
+int edk_internal_pinned(edk_ctx *ctx, size_t doubles, double **buf, cudaEvent_t *ev)
+{
+    const int rc = ensure_pinned(ctx, doubles);
+    *buf = ctx->pin_tri;
+    *ev = ctx->pin_ev;
+    return rc;
+}
 
 edk_ctx *edk_internal_h_ctx(edk_h *h) { return h->ctx; }
 

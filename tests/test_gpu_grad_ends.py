@@ -1,6 +1,6 @@
 """Ends of the adjoint's recurrences: a right-hand side that vanishes (a sector of
-one state), and more frequencies than the continued fraction's buffers hold at a
-time."""
+one state), a chain that breaks down long before its last step, and more
+frequencies than the continued fraction's buffers hold at a time."""
 import numpy as np
 import pytest
 
@@ -33,6 +33,23 @@ def test_one_state_has_no_residual(ctx):
     grad, G, st = h.grad_green(_unit(1, 0), 0.0, [(0, 0, True)], 5, wn, gbar, edk.star_params(m))
     assert st["cg_iterations"] == 0 and st["cg_residual"] == 0.0
     assert np.isfinite(grad).all() and np.isfinite(G).all()
+
+
+def test_chain_stops_soon_after_a_breakdown(ctx):
+    """No hybridisation: c+|basis state> is an eigenstate and the chain ends after one
+    step.  The launches of a call do not grow with the steps it was allowed."""
+    m = star_model(-1.0, 2.0, np.linspace(-0.9, 0.8, 9), np.zeros(9))
+    h = edk.Hamiltonian(ctx, m, 5, 5)
+    wn, params = matsubara(10.0, 8), edk.star_params(m)
+    psi, gbar = _unit(h.dim, 0), np.ones((1, 8), complex)     # the impurity is the highest orbital: empty in state 0
+    e0, out = float(h.hmult(psi)[0]), []
+    for steps in (4, 4, 800):
+        n0 = ctx.launches
+        grad, G, st = h.grad_green(psi, e0, [(0, 0, True)], steps, wn, gbar, params)
+        out.append((grad, G, st["forward_steps"], ctx.launches - n0))
+    assert [o[2] for o in out] == [1, 1, 1]
+    assert np.array_equal(out[1][0], out[2][0]) and np.array_equal(out[1][1], out[2][1])
+    assert out[2][3] <= out[1][3] + 4 * 3 * 45                # at most three segments of sqrt(2 * 800) + 1 steps
 
 
 def test_many_frequencies_need_no_more_memory(ctx):
