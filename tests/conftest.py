@@ -22,3 +22,11 @@ def ctx():
     c = edk.Context(0)
     yield c
     c.close()
+
+
+@pytest.fixture(autouse=True)
+def _default_launch_mode(request):
+    """The session's context leaves every test in the launch mode that users get."""
+    yield
+    if "ctx" in request.fixturenames:
+        request.getfixturevalue("ctx").set_graphs(False)
