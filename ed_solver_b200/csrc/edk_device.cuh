@@ -185,27 +185,6 @@ __device__ __forceinline__ void st1(double *p, double a, uint64_t pol)
 {
     asm volatile("st.global.L2::cache_hint.f64 [%0], %1, %2;" :: "l"(p), "d"(a), "l"(pol) : "memory");
 }
-// The same through the read-only path, for kernels that are launched plainly (the
-// grid before them has ended) and vectors that they do not write themselves.
-__device__ __forceinline__ float ldr1(const float *p, uint64_t pol)
-{
-    float v;
-    asm volatile("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
-    return v;
-}
-__device__ __forceinline__ float2 ldr2(const float *p, uint64_t pol)
-{
-    float2 v;
-    asm volatile("ld.global.nc.L2::cache_hint.v2.f32 {%0,%1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(p), "l"(pol));
-    return v;
-}
-__device__ __forceinline__ float4 ldr4(const float *p, uint64_t pol)
-{
-    float4 v;
-    asm volatile("ld.global.nc.L2::cache_hint.v4.f32 {%0,%1,%2,%3}, [%4], %5;"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(pol));
-    return v;
-}
 __device__ __forceinline__ void prefetch_l2(const void *p)
 {
     asm volatile("prefetch.global.L2::evict_last [%0];" :: "l"(p));

@@ -25,6 +25,29 @@
 
 namespace edk {
 
+// Loads through the read-only path, which the chained kernels must keep off: these
+// kernels are launched plainly (the grid before them has ended) and read vectors
+// that they do not write themselves.
+__device__ __forceinline__ float ldr1(const float *p, uint64_t pol)
+{
+    float v;
+    asm volatile("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
+    return v;
+}
+__device__ __forceinline__ float2 ldr2(const float *p, uint64_t pol)
+{
+    float2 v;
+    asm volatile("ld.global.nc.L2::cache_hint.v2.f32 {%0,%1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(p), "l"(pol));
+    return v;
+}
+__device__ __forceinline__ float4 ldr4(const float *p, uint64_t pol)
+{
+    float4 v;
+    asm volatile("ld.global.nc.L2::cache_hint.v4.f32 {%0,%1,%2,%3}, [%4], %5;"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(pol));
+    return v;
+}
+
 __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c)
 {
     unsigned long long d;

@@ -29,6 +29,7 @@ def test_vectors_keep_off_the_read_only_path(name):
     s = _source(name)
     assert "launch_chained" in s or name.endswith(".cuh")
     assert ".nc" not in "".join(re.findall(r'asm volatile\(\s*"ld[^"]*"', s))
+    assert not re.search(r"\bldr[124]\(", s)              # the plainly launched kernels' loads
     for m in re.finditer(r"__ldg\(\s*(?:reinterpret_cast<[^>]*>\()?(\w+)", s):
         kinds = re.findall(r"(\w+) \*(?:__restrict__ )?%s\b" % m.group(1), s[:m.start()])
         assert not kinds or kinds[-1] not in ("T", "int4"), m.group(0)
