@@ -23,6 +23,7 @@ is not reproducible, so its exact Lanczos coefficient sequence is unpinned.
 from __future__ import annotations
 
 import ctypes as C
+import itertools
 import math
 import os
 import subprocess
@@ -915,3 +916,69 @@ def chiloc_inputs(model: AIMModel, nup: int, ndn: int, site: int = 0):
         CV = np.stack(cols, axis=1)                     # c+ V_s in the target's Fock basis
         M[m] = V[t].T @ CV                               # target x source
     return E, M, V
+
+
+# ---------------------------------------------------------------------------
+# chi~_loc once more, from the published Lehmann sum and not from a list of terms:
+# <T c_1 c+_1 c_2 c+_2> by its six time orders (Hafermann, Krivenko, Rubtsov,
+# Lichtenstein, Katsnelson, EPL 85, 27007 (2009), eq. 23 and its vanishing
+# denominators).  chi_tilde_loc_ gives the part of the sum that carries the
+# Boltzmann factors of one sector: the state of that sector stands at each of the
+# four places in turn.
+# ---------------------------------------------------------------------------
+
+def _lehmann_coefficient(place, beta, w, Ea, Eb, Ec, Ed, eps):
+    """Coefficient of exp(-beta E_place), and the sum of its parts' magnitudes."""
+    w1, w2, w3 = w
+    a = 1.0 / (w3 + Ec - Ed)
+    z1, zb = w1 + Ea - Eb, w2 + Eb - Ec
+    z2, y = w2 + w3 + Eb - Ed, w1 + w2 + Ea - Ec
+    z, inv = w1 + w2 + w3 + Ea - Ed, lambda v: 1.0 / np.where(np.abs(v) > eps, v, 1.0)
+    nz2, ny = np.abs(z2) > eps, np.abs(y) > eps
+    if place == 0:
+        parts = [np.where(nz2, inv(z2) / z1, 1.0 / z1**2), np.where(nz2, -inv(z2) / z, 0.0), -1.0 / (zb * z1),
+                 np.where(ny, inv(y), -beta) / zb]
+    elif place == 1:
+        parts = [np.where(nz2, inv(z2) / z1, 1.0 / z1**2), np.where(nz2, 0.0, -beta / z1), -1.0 / (zb * z1)]
+    elif place == 2:
+        parts = [np.where(ny, -inv(y), 0.0) / zb]
+    else:
+        parts = [np.where(nz2, -inv(z2) / z, 0.0)]
+    return a * sum(parts), np.abs(a) * sum(np.abs(p) for p in parts)
+
+
+def chiloc_lehmann(op, w, phi_eps, beta, Z, gs_e, E, M):
+    """chi~_loc of one sector for one frequency triple (op 1: DNDN, 2: UPDN), and the
+    sum of the magnitudes of all that was added up, which bounds its rounding."""
+    slot = {s: q for q, s in enumerate(CHILOC_SECTORS)}
+    step = [(1, 0), (0, 1)]
+    first = 1 if op == 1 else 0
+    ops = [(first, -1), (first, 1), (1, -1)]             # (spin, change from right to left)
+    total, scale = 0j, 0.0
+    for perm in itertools.permutations(range(3)):
+        sign = 1 if perm in ((0, 1, 2), (1, 2, 0), (2, 0, 1)) else -1
+        chain = [ops[p] for p in perm] + [(1, 1)]
+        for place in range(4):
+            # sectors of the four states: the right neighbour of an operator has what it adds less
+            at = [None] * 4
+            cur = (0, 0)
+            for q in range(4):
+                at[(place + q) % 4] = cur
+                sp, d = chain[(place + q) % 4]
+                cur = (cur[0] - d * step[sp][0], cur[1] - d * step[sp][1])
+            idx = [slot.get(s) for s in at]
+            if any(q is None or E[q] is None for q in idx):
+                continue
+            fac = []
+            for q, (sp, d) in enumerate(chain):
+                left, right = idx[q], idx[(q + 1) % 4]
+                key = (left, right, sp) if d == 1 else (right, left, sp)
+                m = M[CHILOC_MATRICES.index(key)]
+                fac.append(m if d == 1 else m.T)
+            me = np.einsum("ab,bc,cd,da->abcd", *fac)
+            Es = [np.asarray(E[q]).reshape([-1 if r == q2 else 1 for r in range(4)]) for q2, q in enumerate(idx)]
+            c, mag = _lehmann_coefficient(place, beta, [w[p] for p in perm], *Es, phi_eps)
+            boltz = np.exp(-beta * (Es[place] - gs_e)) / Z
+            total += sign * complex((me * c * boltz).sum())
+            scale += float((np.abs(me) * mag * boltz).sum())
+    return total, scale
