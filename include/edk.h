@@ -82,7 +82,7 @@ int edk_ctx_timing(edk_ctx *ctx, int enable);
  * the same shape), 1 = always the generic kernel (for A/B checks), 2 or 3 = the
  * fast kernel where its preconditions hold with its default launch shape,
  * 16+i (i < 32) = the fast kernel with its i-th feasible launch shape (modulo
- * their number), for measurements. */
+ * their number), for measurements; batched chains likewise. */
 int edk_ctx_set_kernel_path(edk_ctx *ctx, int path);
 /* 0 (default): Lanczos passes and Green chains launch each fused step, which
  * overlaps its tables with the end of the step before; 1: pairs of fused steps
