@@ -335,9 +335,9 @@ struct edk_h {
     };
     std::vector<std::unique_ptr<CMap>> cmaps;
     // fast-kernel launch shape per element type, chosen by timing on first use
-    // (index: element type + 2 * FP32 hop sums)
-    FastShape fast_shape[4];
-    bool fast_tuned[4] = {false, false, false, false};
+    // (index: shape_slot)
+    FastShape fast_shape[8];
+    bool fast_tuned[8] = {};
     // Nambu (Sz) sector: its tables replace the (N_up, N_dn) ones
     SzHost *sz = nullptr;
     int npart = -1;
@@ -467,13 +467,18 @@ int sum32_for(const edk_h *h, int dtype)
 }
 
 // What a timed launch shape is kept under: all that the candidates depend on.
-std::string shape_key(const edk_h *h, int dtype, int sum32)
+std::string shape_key(const edk_h *h, int dtype, int sum32, bool hv)
 {
     char key[160];
-    std::snprintf(key, sizeof key, "%d:%lld:%lld:%d:%d:%d:%d:%d", dtype, (long long)h->H.dup, (long long)h->H.ddn,
-                  h->H.up.ell_k, h->H.dn_kmax, h->H.nc, sum32, h->H.hund);
+    std::snprintf(key, sizeof key, "%d:%lld:%lld:%d:%d:%d:%d:%d:%d", dtype, (long long)h->H.dup, (long long)h->H.ddn,
+                  h->H.up.ell_k, h->H.dn_kmax, h->H.nc, sum32, h->H.hund, hv);
     return key;
 }
+
+// Index of edk_h::fast_shape.  Plain H*v has a shape of its own: the one that is
+// fastest for a fused step can be a quarter slower for it (853,776 states with Hund
+// terms: steps of 37.2 to 38.6 us whose shapes take 21.4 to 26.8 us per H*v).
+int shape_slot(int dtype, int sum32, bool hv) { return dtype + 2 * sum32 + (hv ? 4 : 0); }
 
 // aligned: every vector of the call is aligned to twice the element size,
 // which the register-staged kernel (kind 0) needs; without it only the
@@ -483,7 +488,8 @@ int fast_shape_for(edk_h *h, int dtype, const RowArgs &a, bool aligned, FastShap
     edk_ctx *c = h->ctx;
     const int eb = dtype == EDK_F64 ? 8 : 4;
     FastShape cand[kMaxShapes];
-    const int slot = dtype + 2 * a.sum32;
+    const bool hv = a.mode == kModeHv;
+    const int slot = shape_slot(dtype, a.sum32, hv);
     if (c->kernel_path >= 16) {
         // a fixed candidate, for measurements
         const int n = fast_shapes(h->H, eb, c->num_sms, cand, kMaxShapes, a.sum32);
@@ -500,27 +506,38 @@ int fast_shape_for(edk_h *h, int dtype, const RowArgs &a, bool aligned, FastShap
         out = cand[0];
         return EDK_OK;
     }
-    const std::string key = shape_key(h, dtype, a.sum32);
-    if (c->kernel_path == 0)
+    // kept by another handle of the sector's shape
+    auto kept = [&](const std::string &k) -> const FastShape * {
         for (const auto &kv : c->fast_by_shape)
-            if (kv.first == key) {
-                out = h->fast_shape[slot] = kv.second;
-                h->fast_tuned[slot] = true;
-                return EDK_OK;
-            }
+            if (kv.first == k) return &kv.second;
+        return nullptr;
+    };
+    const std::string key = shape_key(h, dtype, a.sum32, hv);
+    if (c->kernel_path == 0)
+        if (const FastShape *f = kept(key)) {
+            out = h->fast_shape[slot] = *f;
+            h->fast_tuned[slot] = true;
+            return EDK_OK;
+        }
     const int n = fast_shapes(h->H, eb, c->num_sms, cand, kMaxShapes, a.sum32);
     if (n == 0) return c->fail(EDK_ERR_INVALID, "fast row kernel: no launch shape");
     out = cand[0];
-    // inside a caller's capture nothing can be timed: a later call does it
+    // inside a caller's capture nothing can be timed: a later call does it.  H*v takes
+    // the steps' shape there if it is known.
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(c->stream, &capture) != cudaSuccess) (void)cudaGetLastError();
-    if (capture != cudaStreamCaptureStatusNone) return EDK_OK;
+    if (capture != cudaStreamCaptureStatusNone) {
+        const int step = shape_slot(dtype, a.sum32, false);
+        if (h->fast_tuned[step]) out = h->fast_shape[step];
+        else if (const FastShape *f = kept(shape_key(h, dtype, a.sum32, false))) out = *f;
+        return EDK_OK;
+    }
     if (c->kernel_path != 0 || n == 1 || !a.x || !a.y) {
         if (n == 1 || c->kernel_path != 0) { h->fast_shape[slot] = out; h->fast_tuned[slot] = true; }
         return EDK_OK;
     }
-    // Candidates are timed as the launch they mostly serve, a fused Lanczos
-    // step, against scratch coefficients, flags and reduction buffers of their
+    // H*v is timed as it is.  For the other modes candidates are timed as the launch
+    // they mostly serve, a fused Lanczos step, against scratch coefficients, flags and reduction buffers of their
     // own (so the live Lanczos state is untouched) and a zeroed scratch vector
     // that stands in for v_k, v_{k-1} and the second output: x is gathered,
     // the call's y is written (the real launch then overwrites it).  The
@@ -530,7 +547,7 @@ int fast_shape_for(edk_h *h, int dtype, const RowArgs &a, bool aligned, FastShap
     t.mode = kModeHv;
     DevBuf tv, tstate;
     const size_t vbytes = (size_t)h->dim * eb;
-    if (tv.ensure(vbytes) == cudaSuccess && tstate.ensure(sizeof(double) * (16 + 4 * (size_t)c->num_sms * 16) + 256) ==
+    if (!hv && tv.ensure(vbytes) == cudaSuccess && tstate.ensure(sizeof(double) * (16 + 4 * (size_t)c->num_sms * 16) + 256) ==
                                                 cudaSuccess) {
         double *tri = tstate.as<double>();                 // tri_diag [0..7], tri_sub [8..15]
         double *part = tri + 16;
@@ -557,7 +574,7 @@ int fast_shape_for(edk_h *h, int dtype, const RowArgs &a, bool aligned, FastShap
         t.vout = tv.p;
         t.psi = nullptr;
         t.psi_coef = nullptr;
-    } else {
+    } else if (!hv) {
         (void)cudaGetLastError();
     }
     // each candidate: one warm-up launch, then the best of three timed ones
@@ -1489,14 +1506,17 @@ int edk_h_launch_shape_chosen(const edk_h *h, int dtype, int fp32_sums, int32_t 
     if (!h || !desc || (dtype != EDK_F64 && dtype != EDK_F32)) return EDK_ERR_INVALID;
     if (h->sz) return 0;
     const int s32 = dtype == EDK_F32 && fp32_sums ? 1 : 0;
-    const int slot = dtype + 2 * s32;
+    // the fused step's, else plain H*v's
     FastShape out;
     bool found = false;
-    if (h->fast_tuned[slot]) {
-        out = h->fast_shape[slot];
-        found = true;
-    } else {
-        const std::string key = shape_key(h, dtype, s32);
+    for (int hv = 0; hv < 2 && !found; ++hv) {
+        const int slot = shape_slot(dtype, s32, hv != 0);
+        if (h->fast_tuned[slot]) {
+            out = h->fast_shape[slot];
+            found = true;
+            continue;
+        }
+        const std::string key = shape_key(h, dtype, s32, hv != 0);
         for (const auto &kv : h->ctx->fast_by_shape)
             if (kv.first == key) { out = kv.second; found = true; }
     }

@@ -78,9 +78,9 @@ int64_t edk_ctx_launch_count(const edk_ctx *ctx);
 int edk_ctx_timing(edk_ctx *ctx, int enable);
 /* Row-kernel selection: 0 = the fastest kernel whose preconditions hold
  * (default; the fast kernel's launch shape is timed once per sector shape
- * and element type, and the context keeps the choice for later Hamiltonians of
- * the same shape), 1 = always the generic kernel (for A/B checks), 2 or 3 = the
- * fast kernel where its preconditions hold with its default launch shape,
+ * and element type, for plain H*v and for the fused steps each on its first
+ * call, and the context keeps the choice for later Hamiltonians of the same
+ * shape), 1 = always the generic kernel (for A/B checks), 2 or 3 = the fast kernel where its preconditions hold with its default launch shape,
  * 16+i (i < 32) = the fast kernel with its i-th feasible launch shape (modulo
  * their number), for measurements; batched chains likewise. */
 int edk_ctx_set_kernel_path(edk_ctx *ctx, int path);
@@ -160,9 +160,9 @@ int edk_h_launch_shapes(const edk_h *h, int dtype, int32_t *desc, int32_t cap);
 /* The launch shape the timing chose for this sector shape and element type
  * (with fp32_sums != 0: for FP32 hop sums): 1 and the 5 ints of
  * edk_h_launch_shapes in desc when one was chosen on this handle or on
- * another handle of the same sector shape in the context, 0 when none has
- * been, EDK_ERR_INVALID on bad arguments.  No counterpart in the reference
- * (a report of this library's own launch-shape tuning). */
+ * another handle of the same sector shape in the context (the fused steps',
+ * or plain H*v's where no step has run), 0 when none has been,
+ * EDK_ERR_INVALID on bad arguments.  No counterpart in the reference (a report of this library's own launch-shape tuning). */
 int edk_h_launch_shape_chosen(const edk_h *h, int dtype, int fp32_sums, int32_t *desc);
 /* Export one spin species' table (tab_HAIM2, HAIM_offdiag_arrays.f90:210-606)
  * as built for the device: CSR row pointer ptr[dim_s+1], 0-based target rank
