@@ -358,11 +358,13 @@ __global__ void __launch_bounds__(256, 4) down_pass_kernel(const HamDev H, const
                     const double wd = (double)wt[e];
                     s0 += wd * wd; s1 += wd * vd; s2 += vd * vd;
                 }
+                // before the stores (see row_lean_kernel)
+                float2 pv = make_float2(0.f, 0.f);
+                if (a.psi) pv = ld2(static_cast<const float *>(a.psi) + i, stream);
                 st2(static_cast<float *>(a.y) + i, wt[0], wt[1], stream);
                 st2(static_cast<float *>(a.vout) + i, vt[0], vt[1], stream);
                 if (a.psi) {
                     float *p = static_cast<float *>(a.psi) + i;
-                    const float2 pv = ld2(p, stream);
                     st2(p, (float)((double)pv.x + sc.cpsi * (double)vt[0]), (float)((double)pv.y + sc.cpsi * (double)vt[1]),
                         stream);
                 }
@@ -478,11 +480,13 @@ __global__ void __launch_bounds__(256, 3) down_pass4_kernel(const HamDev H, cons
                     const double wd = (double)wt[e];
                     s0 += wd * wd; s1 += wd * vd; s2 += vd * vd;
                 }
+                // before the stores (see row_lean_kernel)
+                float4 pv = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (a.psi) pv = ld4(static_cast<const float *>(a.psi) + i, stream);
                 st4(static_cast<float *>(a.y) + i, wt[0], wt[1], wt[2], wt[3], stream);
                 st4(static_cast<float *>(a.vout) + i, vt[0], vt[1], vt[2], vt[3], stream);
                 if (a.psi) {
                     float *p = static_cast<float *>(a.psi) + i;
-                    const float4 pv = ld4(p, stream);
                     st4(p, (float)((double)pv.x + sc.cpsi * (double)vt[0]), (float)((double)pv.y + sc.cpsi * (double)vt[1]),
                         (float)((double)pv.z + sc.cpsi * (double)vt[2]), (float)((double)pv.w + sc.cpsi * (double)vt[3]),
                         stream);
