@@ -13,6 +13,13 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (B200); runs the CUDA path")
 
 
+def pytest_collection_modifyitems(items):
+    """Tests that want the reference's compiled code come last: where its source is absent
+    they fail, and a run that stops at the first failure has then run all the others."""
+    wants_ref = lambda i: "_need_ref" in i.function.__code__.co_names
+    items.sort(key=wants_ref)
+
+
 @pytest.fixture(scope="session")
 def ctx():
     import torch
