@@ -496,8 +496,12 @@ __global__ void __launch_bounds__(kChiBlock, 3) chi_terms_hoisted_kernel(const C
 // One block per (term, triple), its tables in shared memory (five of n (n | 1)
 // complex numbers, 107 KB at n = 36: two blocks per SM) or, for larger
 // sectors, in a slice of global memory; a thread owns two states i and one of
-// the cycle's other indices, so one table element serves both states.  FP64
-// arithmetic and shared-memory loads bound it about equally.
+// the cycle's other indices, so one table element serves both states.  What
+// bounds it: the L1 data pipe (67 % full, FP64 22 %, issue 41 % at n = 36), with
+// the tables' loads, the strided loads of the outer factors and the barriers
+// between the stages of a term.  Tables in global memory (L2) cost little more: 512
+// triples at n = 100 take 55 ms, 1.2 times what n^3 gives from n = 36; 32 of them 5.9,
+// with the split kernel 871.
 struct FacTerm {
     int op, nphi, kind[2], perm[2][3], sgn[2], total;
     int sx, sm, sy;           // sectors of x, m, y

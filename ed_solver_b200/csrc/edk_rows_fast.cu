@@ -52,7 +52,7 @@ int fast_shapes(const HamDev &H, int elem_bytes, int num_sms, FastShape *out, in
         // Hund terms: kinds 1 and 2, as many blocks per SM as the staged rows allow
         // (two buffers a block and up to 5.5 KB of tables).  FP64 H*v of two-orbital
         // sectors, us, against the generic row kernel's: 2,944,656 states 66 (kind 2,
-        // 128 threads; 73 kind 1) / 137; 853,776 24 / 46; 213,444 9.6 / 17.2; FP32
+        // 128 threads; 73 kind 1) / 137; 853,776 21.4 / 46; 213,444 9.6 / 17.2; FP32
         // 2,944,656 47 / 124.  Below 2^17 states the shapes lie within the timing's
         // noise (63,504: 5.1-5.5, generic 5.5), so one is taken untimed.
         const int kmax = H.up.ell_k > H.dn_kmax ? H.up.ell_k : H.dn_kmax;

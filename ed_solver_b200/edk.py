@@ -471,7 +471,8 @@ class Hamiltonian:
 
     def launch_shape_chosen(self, dtype="f32", fp32_sums=True):
         """The launch shape the timing chose for this sector shape (a dict as
-        in launch_shapes), or None when none has been chosen yet."""
+        in launch_shapes): the fused steps', or plain H*v's where no step has run;
+        None when none has been chosen yet."""
         desc = np.zeros(5, np.int32)
         rc = lib().edk_h_launch_shape_chosen(self.h, _dtype_code(dtype), int(bool(fp32_sums)), desc.ctypes.data)
         if rc < 0:
@@ -805,7 +806,8 @@ def chiloc(ctx: Context, E, M, w, beta: float, Z: float, gs_e: float, sites: int
 
 
 def chiloc_set_kernel(plain: bool):
-    """edk_chiloc's kernel: False = the split kernel (default), True = the per-element one."""
+    """edk_chiloc's kernel: False = the factored kernel, or the split one where it does not
+    apply (default), True = the per-element one."""
     lib().edk_chiloc_set_kernel(int(bool(plain)))
 
 

@@ -80,9 +80,10 @@ int edk_ctx_timing(edk_ctx *ctx, int enable);
  * (default; the fast kernel's launch shape is timed once per sector shape
  * and element type, for plain H*v and for the fused steps each on its first
  * call, and the context keeps the choice for later Hamiltonians of the same
- * shape), 1 = always the generic kernel (for A/B checks), 2 or 3 = the fast kernel where its preconditions hold with its default launch shape,
- * 16+i (i < 32) = the fast kernel with its i-th feasible launch shape (modulo
- * their number), for measurements; batched chains likewise. */
+ * shape), 1 = always the generic kernel (for A/B checks), 2 or 3 = the fast
+ * kernel where its preconditions hold with its default launch shape, 16+i
+ * (i < 32) = the fast kernel with its i-th feasible launch shape (modulo their
+ * number), for measurements; batched chains likewise. */
 int edk_ctx_set_kernel_path(edk_ctx *ctx, int path);
 /* 0 (default): Lanczos passes and Green chains launch each fused step, which
  * overlaps its tables with the end of the step before; 1: pairs of fused steps
@@ -104,7 +105,10 @@ int edk_ctx_clear_cache(edk_ctx *ctx);
 /* Hands the device memory that the context's Krylov-basis pool keeps in
  * reserve (released bases, up to 5/8 of the device) back to the driver, so
  * that other allocators can use it.  The next pass that keeps its basis maps
- * memory again.  Nothing else is freed. */
+ * memory again.  Also frees what the other calls keep between calls: up to 1 GB
+ * of that pool after a gradient, and the local vertex's scratch, three buffers
+ * of up to 256 MB each.  Nothing else is freed.  Waits for the context's
+ * stream. */
 int edk_ctx_trim(edk_ctx *ctx);
 /* Caps the Krylov workspace (five vectors of the sector's size per element
  * type, shared by the context's passes): a pass that would need more than
@@ -162,7 +166,8 @@ int edk_h_launch_shapes(const edk_h *h, int dtype, int32_t *desc, int32_t cap);
  * edk_h_launch_shapes in desc when one was chosen on this handle or on
  * another handle of the same sector shape in the context (the fused steps',
  * or plain H*v's where no step has run), 0 when none has been,
- * EDK_ERR_INVALID on bad arguments.  No counterpart in the reference (a report of this library's own launch-shape tuning). */
+ * EDK_ERR_INVALID on bad arguments.  No counterpart in the reference (a report
+ * of this library's own launch-shape tuning). */
 int edk_h_launch_shape_chosen(const edk_h *h, int dtype, int fp32_sums, int32_t *desc);
 /* Export one spin species' table (tab_HAIM2, HAIM_offdiag_arrays.f90:210-606)
  * as built for the device: CSR row pointer ptr[dim_s+1], 0-based target rank
@@ -343,7 +348,10 @@ typedef struct edk_batch_stats {
     int64_t steps;               /* Lanczos steps run over all chains */
     int32_t chains;
     double kernel_ms;            /* device time of the persistent launch */
-    int32_t block, rows, blocks_per_sm, tuned_shapes;
+    int32_t block;               /* threads per block */
+    int32_t rows;                /* rows a thread sums at a time: 1 */
+    int32_t blocks_per_sm;       /* blocks launched per SM, at least 1 */
+    int32_t tuned_shapes;        /* launch shapes this call timed (0: kept from before) */
 } edk_batch_stats;
 
 int edk_green_batch(edk_ctx *ctx, int dtype, int32_t nchain, const edk_chain *chains, int32_t nitergreen,
@@ -627,10 +635,12 @@ typedef struct edk_chiloc_sectors {
 int edk_chiloc(edk_ctx *ctx, int32_t op_mask, double beta, double Z, double gs_e, double phi_eps, int32_t sites,
                int32_t nup, int32_t ndn, const edk_chiloc_sectors *s, int32_t nf, const double *w_host,
                double *pdndn_host, double *pupdn_host);
-/* Process-wide kernel choice of edk_chiloc: 0 (default) = the kernel that
- * computes the one-index parts of the Phi coefficients once per block (when
- * they fit in 96 KB of shared memory), 1 = the per-element kernel, for A/B
- * checks. */
+/* Process-wide kernel choice of edk_chiloc: 0 (default) = the factored kernel,
+ * which contracts the four-fold sum pairwise; a call with a frequency w1, w2, w3
+ * or w1 + w2 + w3 within 1e-8 of the real axis, or without room for its tables,
+ * takes the split kernel, which computes the one-index parts of the Phi
+ * coefficients once per block (when they fit in 96 KB of shared memory); 1 = the
+ * per-element kernel, for A/B checks. */
 int edk_chiloc_set_kernel(int plain);
 
 #ifdef __cplusplus
