@@ -452,8 +452,8 @@ RowArgs base_args(edk_h *h)
 }
 
 // The fast kernel's launch shape for this sector and element type.  On the
-// first call with an output vector, every feasible shape is timed (four
-// launches each, the first as warm-up, the best of the other three counted)
+// first call with an output vector, every feasible shape is timed (a warm-up launch,
+// then the best of three: single launches, or a few in a row of a short kernel)
 // writing into that vector, which the real launch then overwrites; the
 // fastest is kept on the Hamiltonian.
 constexpr int kMaxShapes = 32;
@@ -562,7 +562,7 @@ int fast_shape_for(edk_h *h, int dtype, const RowArgs &a, bool aligned, FastShap
         t.k = 1;
         t.kdev = nullptr;
         t.gamma1 = 0.0;
-        t.cutoff = 1e-300;
+        t.cutoff = 0.0;                                    // launches in a row: none ends the chain
         t.tri_diag = tri;
         t.tri_sub = tri + 8;
         t.partials = part;
@@ -577,22 +577,33 @@ int fast_shape_for(edk_h *h, int dtype, const RowArgs &a, bool aligned, FastShap
     } else if (!hv) {
         (void)cudaGetLastError();
     }
-    // each candidate: one warm-up launch, then the best of three timed ones
-    // (a single timed launch let clock and cache noise pick a shape 40 % slower)
+    // each candidate: one warm-up launch, then the best of three timed ones (a single
+    // timed launch let clock and cache noise pick a shape 40 % slower).  Kernels below
+    // 60 us are timed eight in a row, as a chain runs them: of one launch alone the
+    // events' and the start's own time is half, and its noise picked other shapes from
+    // context to context: steps of 13.6 to 15.2 us at 152,460 states with Hund terms
+    // (13.5 now), 33.3 to 35.5 at 853,776 (33.0), 7.0 to 8.2 at 4,900 (7.0), 12.1 to
+    // 12.7 at 213,444 (11.7).  It takes 1 to 2 ms more per sector shape, once.
     cudaEvent_t ea = c->get_event(), eb_ = c->get_event();
     float best = 3.0e38f;
     for (int i = 0; i < n; ++i) {
         float cbest = 3.0e38f;
+        int row = 1;
         for (int rep = 0; rep < 4; ++rep) {
             if (t.mode == kModeStep) cudaMemsetAsync(reinterpret_cast<void *>(t.counter), 0, 256, c->stream);
             cudaEventRecord(ea, c->stream);
-            cudaError_t e = launch_rows_fast(h->H, dtype, t, c->num_sms, cand[i], c->stream);
+            cudaError_t e = cudaSuccess;
+            for (int q = 0; q < row && e == cudaSuccess; ++q, c->launches++)
+                e = launch_rows_fast(h->H, dtype, t, c->num_sms, cand[i], c->stream);
             cudaEventRecord(eb_, c->stream);
-            c->launches++;
             if (e != cudaSuccess) { (void)cudaGetLastError(); cbest = 3.0e38f; break; }
             float ms = 0.f;
             if (cudaEventSynchronize(eb_) != cudaSuccess || cudaEventElapsedTime(&ms, ea, eb_) != cudaSuccess) break;
-            if (rep >= 1 && ms < cbest) cbest = ms;
+            if (rep == 1 && ms < 0.06f) {      // (the first launch may have loaded the kernel)
+                row = 8;
+                continue;
+            }
+            if (rep >= 1) cbest = std::min(cbest, ms / row);
         }
         if (cbest < best) { best = cbest; out = cand[i]; }
     }

@@ -47,6 +47,28 @@ def test_each_mode_is_timed_once(first, ns, nc, sec):
         c.close()
 
 
+@pytest.mark.parametrize("ns,sec", [(8, (4, 4)), (11, (6, 5))])
+def test_first_chain_ends_at_once(ns, sec):
+    """The shapes are timed on a vector whose Krylov space is itself: no step of the timing
+    may take the chain for ended."""
+    import torch
+    m = star_model([-1.2], 2.5, np.linspace(-1.5, 1.5, ns - 1), np.zeros(ns - 1))
+    wn, out = matsubara(20.0, 8), []
+    for path in (0, 1):
+        c = edk.Context(0)
+        try:
+            h = edk.Hamiltonian(c, m, *sec)
+            c.set_kernel_path(path)
+            x = torch.zeros(h.dim, dtype=torch.float64, device="cuda")
+            x[h.dim // 3] = 1.0
+            out.append(h.green_chain(x, 5, -3.0, 1, wn)[0])
+            e = float(h.hmult(x)[h.dim // 3])
+        finally:
+            c.close()
+        assert np.abs(out[-1] - 1.0 / (1j * wn - (e + 3.0))).max() <= 1e-12
+    assert np.array_equal(out[0], out[1])
+
+
 @pytest.mark.parametrize("same", [True, False])
 def test_capture_after_steps_is_not_timed(same):
     import torch
